@@ -72,7 +72,25 @@ def _cut(rng, total, most):
     return ",".join(str(s) for s in sizes)
 
 
+def _like_sized(case):
+    """Whether the contracted block pairs of a modular case are all long (about
+    a thousand elements) or all short, as blocks of like size give."""
+    o, v = ([int(x) for x in case[k].split(",")] for k in ("occ", "vir"))
+    for op, left in (("ladder", v), ("ring", o)):
+        k = [x * y for x in left for y in v]
+        if case["op"] in (op, "ccd") and not (all(x >= 1024 for x in k) or all(x < 1021 for x in k)):
+            return False
+    return True
+
+
 def draw(rng):
+    while True:
+        c = _draw(rng)
+        if c.get("mode") != "modular" or c["op"] == "fock" or _like_sized(c):
+            return c
+
+
+def _draw(rng):
     op = rng.choice(["ladder", "ladder", "ladder", "ladder", "ring", "ring", "fock", "copy", "add", "symm", "dot",
                      "ccd"])
     if op in ("copy", "dot"):
