@@ -55,6 +55,7 @@ constexpr uint64_t kWaitNs = 2000000000ull;         // 2 s: the drain waits afte
 constexpr double kMagicD = 6755399441055744.0;      // 1.5 * 2^52: round-to-integer constant
 constexpr float kMagicF = 12582912.0f;              // 1.5 * 2^23
 constexpr int32_t kNoExp = -1000000;                // exponent of a row with no non-zero element
+constexpr int32_t kKeepRow = -2000000;              // redo pass: a row whose residues stand
 
 // The moduli (pairwise coprime, <= 256) and the constants derived from them,
 // as compile-time functions so that unrolled loops over the moduli fold them
@@ -285,9 +286,11 @@ __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, ui
 // Sampled rows (sampled_panel): their residues are formed with the sampled
 // bound e (|x| < 2^e unless the sample missed the row's largest elements),
 // and the row's exact exponent goes to the side's second table (ext / eyt).
-// With redo set, only those rows run again, and only where the exact
-// exponent exceeds the bound: with the exact exponent, overwriting the
-// residues formed before (whose integers may have exceeded 2^P).
+// With redo set, only the rows of C whose exact exponent exceeds the bound run
+// again, in every panel that feeds them (the sampled ones, whose integers may
+// have exceeded 2^P, and the short ones beside them, which must share the
+// row's scaling): with the exact exponent, overwriting the residues formed
+// before.
 template<int L>
 __global__ void __launch_bounds__(kSplitThreads, 4)
 crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ units, int32_t nunits,
@@ -302,15 +305,22 @@ crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
         const int4 un = units[u];
         const DCrtPanel &P = panels[un.x];
         // tabulated k offsets and the tile mapping's row tables (uniform)
-        const bool shared = P.nk != 1 || P.kstr[0] != 1 || (un.w == kUnitTileMap && !redo);
+        const bool shared = P.nk != 1 || P.kstr[0] != 1 || un.w == kUnitTileMap;
         if (shared) __syncthreads();                         // the previous unit's readers are done
         const int mode = koff_setup(P, koff);
-        if (un.w == kUnitTileMap && !redo)
+        if (un.w == kUnitTileMap)
             for (int i = threadIdx.x; i < un.z; i += blockDim.x) {
                 const int r = un.y + i;
                 const bool valid = r < P.rows;
                 roff[i] = valid ? mixed_offset(r, P.nr, P.rext, P.rstr) : 0;
-                rexp[i] = valid ? (P.side == 0 ? ex : ey)[gidx[P.g_off + r]] : kNoExp;
+                const int g = valid ? gidx[P.g_off + r] : 0;
+                int e = valid ? (P.side == 0 ? ex : ey)[g] : kNoExp;
+                if (redo) {
+                    // kKeepRow: the residues stand as they are
+                    const int et = valid ? (P.side == 0 ? ext : eyt)[g] : kNoExp;
+                    e = et > e ? et : kKeepRow;
+                }
+                rexp[i] = e;
             }
         if (shared) __syncthreads();
         const double *src = (P.src ? B : A) + P.src_off;
@@ -404,7 +414,6 @@ crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
             const int lr = threadIdx.x >> 3, c = threadIdx.x & 7;
             const int r = un.y + lr;
             const bool smp = sample && sampled_panel(P, un.w);       // uniform over the CTA
-            if (redo && !smp) continue;
             const bool rv = lr < un.z && r < P.wrows;
             // largest |x| of the row as the largest high word without its
             // sign bit (ordered as |x|; its exponent field is that of the maximum)
@@ -450,14 +459,13 @@ crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
             }
             continue;
         }
-        if (redo) continue;                                  // tile-mapped units read every element
         const int nkt = (P.wk + 15) >> 4;
         const int ntile = ((un.z + 7) >> 3) * nkt;
         for (int t = warp; t < ntile; t += kSplitWarps) {
             const int rg = t / nkt, kt = t - rg * nkt;
             const int rl = rg * 8 + lrow, r = un.y + rl;
             const int k0 = kt * 16 + kq * 4;
-            if (rl >= un.z || r >= P.wrows || k0 >= P.wk) continue;
+            if (rl >= un.z || r >= P.wrows || k0 >= P.wk || rexp[rl] == kKeepRow) continue;
             if (r != cur) set_row(r, rexp[rl], roff[rl]);
             put4(r, k0);
         }

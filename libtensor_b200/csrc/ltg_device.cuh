@@ -345,8 +345,8 @@ cudaError_t launch_crt_fused(int shape, const DCrtPanel *panels, const DCrtFamil
     const int32_t *famt, const int4 *units, int32_t nunits, const double *a, const double *b,
     const int32_t *gidx, int32_t *ex, int32_t *ey, uint8_t *res, const CrtParams &cp, cudaStream_t s);
 // sample != 0: sampled rows also form their exact exponents into ext / eyt
-// (set to "no element" before); redo != 0: only the sampled rows whose exact
-// exponent exceeds their bound run, with the exact exponent.
+// (set to "no element" before); redo != 0: only the rows whose exact exponent
+// exceeds their bound run, in every panel, with the exact exponent.
 cudaError_t launch_crt_residues(const DCrtPanel *panels, const int4 *units, int32_t nunits,
     const double *a, const double *b, const int32_t *gidx, const int32_t *ex, const int32_t *ey,
     int32_t *ext, int32_t *eyt, int32_t sample, int32_t redo, uint8_t *res, const CrtParams &cp,
