@@ -195,7 +195,7 @@ struct SymExec {
 // Device arrays of the split-precision path for one (C tensor, coefficients,
 // mode, slice count).
 struct OzExec {
-    int kind = 0, S = 0, chunk_kb = 1, npanels = 0, max_rows_pad = 0, nitems = 0;
+    int kind = 0, S = 0, chunk_kb = 1, npanels = 0, max_rows_pad = 0, nitems = 0, swap = 0, max_nt = 16;
     int64_t src_elems = 0, slice_bytes = 0;   // operand elements read, slice bytes written
     DevBuf panels, slices, exps, tasks, cblks, items;
     std::vector<std::pair<int64_t, int64_t>> zero_ranges;
@@ -774,14 +774,23 @@ OzExec *prepare_ozaki(ltg_plan *pl, ltg_bt *c, int mode, int S, double ka, doubl
     std::unique_ptr<OzExec> ex(new OzExec());
     ex->kind = kind;
     ex->S = S;
-    // exact accumulation: S * maxprod * Kc below 2^31 (INT32) or 2^24 (FP32)
-    const int64_t lim = kind == kOzInt8 ? ((int64_t)1 << 31) - 1 : ((int64_t)1 << 24) - 1;
+    // exact accumulation: S * maxprod * Kc below 2^31 (INT32) or up to 2^24 (FP32)
+    const int64_t lim = kind == kOzInt8 ? ((int64_t)1 << 31) - 1 : (int64_t)1 << 24;
     int64_t kc_elems = lim / ((int64_t)S * maxprod);
     ex->chunk_kb = (int)std::max<int64_t>(1, std::min<int64_t>(kc_elems / kbe, 1 << 20));
 
     std::vector<GemmTask> tasks;
     std::vector<CBlockTask> cbt;
     contract2_tasks(pl->plan(), pl->a->h, pl->b->h, c->h, ka, kb, kc, tasks, cbt);
+    // orientation: the C side that gives the cheaper tiling on the MMA M side
+    // (128-row tiles), the other cut into tiles of nt columns
+    double cost_keep = 0, cost_swap = 0;
+    for (const CBlockTask &b : cbt) {
+        cost_keep += b.kflops * oz_product_cost(b.M, b.N, S);
+        cost_swap += b.kflops * oz_product_cost(b.N, b.M, S);
+    }
+    const bool swap = cost_swap < cost_keep;
+    ex->swap = swap ? 1 : 0;
     // panels, de-duplicated by (operand, block, row mapping, k mapping)
     std::map<std::vector<int64_t>, int32_t> pidx;
     std::vector<DPanel> panels;
@@ -799,7 +808,8 @@ OzExec *prepare_ozaki(ltg_plan *pl, ltg_bt *c, int mode, int S, double ka, doubl
         p.src_off = off;
         p.rows = (int32_t)rows.total();
         p.K = (int32_t)k.total();
-        p.rows_pad = (p.rows + 127) / 128 * 128;
+        p.tr = (src == 1) == swap ? 128 : oz_tile_width(p.rows, S);
+        p.rows_pad = (p.rows + p.tr - 1) / p.tr * p.tr;
         p.K_pad = (p.K + 31) / 32 * 32;      // whole 32-element split steps (a multiple of kbe)
         pack_sub(rows, p.nr, p.rext, p.rstr, nullptr);
         SubDims kk = k;
@@ -817,9 +827,11 @@ OzExec *prepare_ozaki(ltg_plan *pl, ltg_bt *c, int mode, int S, double ka, doubl
     std::vector<DOzTask> dt(tasks.size());
     for (size_t i = 0; i < tasks.size(); i++) {
         const GemmTask &t = tasks[i];
-        dt[i].pa = panel_of(0, t.a_off, t.m, t.k, false);
-        dt[i].pb = panel_of(1, t.b_off, t.n, t.k, true);
-        if (panels[dt[i].pa].K_pad != panels[dt[i].pb].K_pad) throw error(kErrState, "panel k extents differ");
+        const int32_t pa = panel_of(0, t.a_off, t.m, t.k, false);
+        const int32_t pb = panel_of(1, t.b_off, t.n, t.k, true);
+        if (panels[pa].K_pad != panels[pb].K_pad) throw error(kErrState, "panel k extents differ");
+        dt[i].px = swap ? pb : pa;
+        dt[i].py = swap ? pa : pb;
     }
     std::vector<DCBlock> dc(cbt.size());
     double post = add ? d : 1.0;
@@ -836,16 +848,19 @@ OzExec *prepare_ozaki(ltg_plan *pl, ltg_bt *c, int mode, int S, double ka, doubl
         x.t_begin = b.t_begin; x.t_end = b.t_end;
         for (int32_t t = b.t_begin; t < b.t_end; t++) dt[t].coeff = tasks[t].coeff / c0;
     }
-    // (C block, 128 x 64 tile) work items, costliest first, dealt round-robin
-    std::vector<std::pair<double, DItem>> iv;
-    for (size_t e = 0; e < cbt.size(); e++)
-        for (int64_t m0 = 0; m0 < cbt[e].M; m0 += 128)
-            for (int64_t n0 = 0; n0 < cbt[e].N; n0 += 64) {
-                DItem it = make_item((int32_t)e, (int32_t)m0, (int32_t)n0);
-                iv.push_back({cbt[e].kflops + 64.0 * (cbt[e].t_end - cbt[e].t_begin), it});
-            }
-    std::stable_sort(iv.begin(), iv.end(), [](const std::pair<double, DItem> &x, const std::pair<double, DItem> &y) { return x.first > y.first; });
-    std::vector<DItem> items;
+    // (C block, 128 x nt tile) work items, costliest first, dealt round-robin
+    std::vector<std::pair<double, DOzItem>> iv;
+    for (size_t e = 0; e < cbt.size(); e++) {
+        const int64_t xe = swap ? cbt[e].N : cbt[e].M, ye = swap ? cbt[e].M : cbt[e].N;
+        const int32_t nt = oz_tile_width(ye, S);
+        ex->max_nt = std::max(ex->max_nt, nt);
+        for (int64_t x0 = 0; x0 < xe; x0 += 128)
+            for (int64_t y0 = 0; y0 < ye; y0 += nt)
+                iv.push_back({nt * (cbt[e].kflops + 64.0 * (cbt[e].t_end - cbt[e].t_begin)),
+                              DOzItem{(int32_t)e, (int32_t)x0, (int32_t)y0, nt}});
+    }
+    std::stable_sort(iv.begin(), iv.end(), [](const std::pair<double, DOzItem> &x, const std::pair<double, DOzItem> &y) { return x.first > y.first; });
+    std::vector<DOzItem> items;
     for (auto &p : iv) items.push_back(p.second);
     for (const DPanel &p : panels) {
         ex->max_rows_pad = std::max(ex->max_rows_pad, p.rows_pad);
@@ -2843,8 +2858,8 @@ int ltg_contract2_symmetrized(ltg_plan *plan, ltg_bt *r, int32_t mode, int32_t n
             t_split.done();
             TimedLaunch t_gemm(ctx, LTG_KERNEL_OZ_GEMM);
             LTG_CUDA(launch_oz_gemm(ox->kind, ox->panels.as<DPanel>(), ox->slices.as<uint8_t>(), ox->tasks.as<DOzTask>(),
-                                    ox->cblks.as<DCBlock>(), ox->items.as<DItem>(), ox->nitems,
-                                    ox->exps.as<int32_t>(), r->arena.as<double>(), 0, ox->S, ox->chunk_kb,
+                                    ox->cblks.as<DCBlock>(), ox->items.as<DOzItem>(), ox->nitems,
+                                    ox->exps.as<int32_t>(), r->arena.as<double>(), 0, ox->S, ox->swap, ox->chunk_kb, ox->max_nt,
                                     ctx->wait_err.as<int32_t>(), ctx->wait_ns, s, ex->drange.as<int2>(),
                                     ex->dests.as<DCBlock>()));
             t_gemm.done();
@@ -3406,8 +3421,8 @@ int ltg_contract2(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nslices, doub
             t_split.done();
             TimedLaunch t_gemm(ctx, LTG_KERNEL_OZ_GEMM);
             LTG_CUDA(launch_oz_gemm(ox->kind, ox->panels.as<DPanel>(), ox->slices.as<uint8_t>(), ox->tasks.as<DOzTask>(),
-                                    ox->cblks.as<DCBlock>(), ox->items.as<DItem>(), ox->nitems,
-                                    ox->exps.as<int32_t>(), c->arena.as<double>(), add, ox->S, ox->chunk_kb,
+                                    ox->cblks.as<DCBlock>(), ox->items.as<DOzItem>(), ox->nitems,
+                                    ox->exps.as<int32_t>(), c->arena.as<double>(), add, ox->S, ox->swap, ox->chunk_kb, ox->max_nt,
                                     ctx->wait_err.as<int32_t>(), ctx->wait_ns, s));
             t_gemm.done();
             ctx->launches += 2;

@@ -73,22 +73,32 @@ enum OzKind { kOzInt8 = 0, kOzBf16 = 1, kOzE4m3 = 2 };
 
 // One split operand panel: the matricised view (rows x K) of a canonical
 // block, cut into S integer-valued slices stored as shared-memory tile images
-// (per row tile, 32-byte k block and slice), rows padded to 128 and K to 32
-// elements.
+// (per tile of tr rows, 32-byte k block and slice), rows padded to whole tiles
+// and K to 32 elements.
 struct DPanel {
     int64_t src_off;              // FP64 source block offset (elements)
     int64_t slice_off;            // byte offset of slice 0 in the slice arena
     int32_t exp_off;              // first row exponent in the exponent arena
     int32_t src;                  // 0: A arena, 1: B arena
     int32_t rows, K, rows_pad, K_pad;
-    int32_t nr, nk;
+    int32_t tr;                   // rows per tile image (128 on the MMA M side, else the N tile width)
+    int32_t nr, nk, pad;
     int32_t rext[kDevMaxSub], rstr[kDevMaxSub];
     int32_t kext[kDevMaxSub], kstr[kDevMaxSub];
 };
 
 struct DOzTask {
-    int32_t pa, pb;               // panels of A and B
+    int32_t px, py;               // panels on the MMA M and N side
     double coeff;                 // relative coefficient of the pair
+};
+
+// One work item of the slice products: the 128 x nt tile of a C block at
+// MMA row x0 and column y0 (rows along the C columns when the sides are
+// swapped).
+struct DOzItem {
+    int32_t cblk;
+    int32_t x0, y0;
+    int32_t nt;
 };
 
 // ---------------------------------------------------------------- CRT (modular) split precision
@@ -316,9 +326,14 @@ cudaError_t launch_oz_split(int kind, const DPanel *panels, int32_t npanels, int
 // added atomically to its destinations (c zeroed before; add ignored); only
 // for each kind's default slice count (INT8 and BF16 7, FP8 8).
 cudaError_t launch_oz_gemm(int kind, const DPanel *panels, const uint8_t *slices, const DOzTask *tasks,
-    const DCBlock *cblks, const DItem *items, int32_t nitems, const int32_t *exps, double *c,
-    int32_t add, int32_t S, int32_t chunk_kb, int32_t *err, uint64_t wait_ns, cudaStream_t s,
-    const int2 *drange = nullptr, const DCBlock *dests = nullptr);
+    const DCBlock *cblks, const DOzItem *items, int32_t nitems, const int32_t *exps, double *c,
+    int32_t add, int32_t S, int32_t swap, int32_t chunk_kb, int32_t max_nt, int32_t *err, uint64_t wait_ns,
+    cudaStream_t s, const int2 *drange = nullptr, const DCBlock *dests = nullptr);
+// Width of the N tiles of an MMA N-side panel of `rows` rows with S slices (a
+// multiple of 16 whose S accumulators fit the tensor memory), and the cost
+// of a product of x by y rows in these tiles (clocks per k block).
+int32_t oz_tile_width(int64_t rows, int S);
+double oz_product_cost(int64_t x, int64_t y, int S);
 // Per kind: first-slice bits, further-slice bits, element bytes, k elements
 // per 64-byte k block, bound of one slice product.
 void oz_kind_params(int kind, int *beta0, int *beta, int *esz, int *kbe, int64_t *maxprod);

@@ -2,9 +2,9 @@
 // generation tensor cores (tcgen05.mma, accumulators in tensor memory).
 //
 // Same schedule and task list as the plain FP64 path (one work item per
-// (C block, 128-row, 64-column) tile, all coalesced pairs of the C block
-// accumulated before the single FP64 write), but the products run on
-// integer-valued low-precision slices:
+// (C block, 128 x nt) tile, all coalesced pairs of the C block accumulated
+// before the single FP64 write), but the products run on integer-valued
+// low-precision slices:
 //
 //  1. split (oz_split_kernel): every matricised operand row r of a block is
 //     scaled by its own power of two 2^-e_r (e_r: exponent of the row's
@@ -24,13 +24,22 @@
 //     into FP64 registers; the C tile is written once, in FP64.
 // Only levels l <= S-1 are formed: S(S+1)/2 slice products per k step.
 //
-// Warp roles (192 threads): warps 0-3 epilogue (TMEM lanes 0-127, one C row
-// per thread), warp 4 bulk-copy producer, warp 5 MMA issuer.  Operand tiles
-// are stored in global memory as the exact shared-memory images the MMA reads
-// (K-major core matrices, no swizzle), so each one moves with a single 1-D
-// cp.async.bulk copy completing on the stage's mbarrier (no tensor maps, no
-// multicast); one MMA k step per pipeline stage, so even 8 slices leave room
-// for 4 stages.
+// The accumulator of level l sits in the nt tensor-memory columns from l * nt,
+// and the N-side image of a k block holds its S slices one after the other, so
+// the products of M-side slice sa with N-side slices 0 .. S-1-sa are one
+// (S - sa) * nt columns wide product into levels sa .. S-1 (issued in pieces of
+// at most 256 columns, the widest MMA).  One MMA per slice pair (nt = 64)
+// reads the M-side slice from shared memory for every 64 columns: 6 KB per
+// 32 clocks of products against 128 B per clock, which held the kernel to a
+// third of the MMA rate (ladder o=40 v=240, BF16 x 4: 8.58 ms).
+//
+// Warp roles (320 threads): warps 0-7 epilogue (two per TMEM lane quarter, one
+// tile row and half of the tile's columns per thread), warp 8 bulk-copy
+// producer, warp 9 MMA issuer.  Operand tiles are stored in global memory as
+// the exact shared-memory images the MMA reads (K-major core matrices, no
+// swizzle), so each one moves with a single 1-D cp.async.bulk copy completing
+// on the stage's mbarrier (no tensor maps, no multicast); one or two MMA k
+// steps per pipeline stage, so even 8 slices leave room for 4 stages.
 // Every mbarrier wait is bounded in time and reports through *err.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
@@ -50,13 +59,20 @@ void oz_kind_params(int kind, int *beta0, int *beta, int *esz, int *kbe, int64_t
 
 namespace {
 
-constexpr int kBM = 128;              // C rows per tile (TMEM lanes)
-constexpr int kBN = 64;               // C columns per tile (TMEM columns per level)
+constexpr int kBM = 128;              // tile rows (TMEM lanes)
 constexpr int kRowBytes = 32;         // k-block row length in shared memory (one MMA k step)
-constexpr int kATile = kBM * kRowBytes;   // 4 KB per A slice per stage
-constexpr int kBTile = kBN * kRowBytes;   // 2 KB per B slice per stage
-constexpr int kThreads = 192;
+constexpr int kXTile = kBM * kRowBytes;   // 4 KB per M-side slice per stage
+constexpr int kEpiWarps = 8;          // two per TMEM lane quarter
+constexpr int kThreads = 32 * (kEpiWarps + 2);
+// Widest N tile: S level accumulators in 512 tensor-memory columns, and at
+// most 64 FP64 sums per epilogue thread.
+__host__ __device__ constexpr int oz_max_nt(int S) { return 512 / S / 16 * 16 < 128 ? 512 / S / 16 * 16 : 128; }
+// Whether the products of M-side slice sa take two MMAs (one is at most 256
+// columns wide; fixed per slice count, so that the issuing loop has no branch).
+template<int S>
+__host__ __device__ constexpr bool two_pieces(int sa) { return (S - sa) * oz_max_nt(S) > 256; }
 constexpr int kMaxStages = 8;
+constexpr int kStageSmem = 200 * 1024;    // shared memory of all stages
 constexpr uint64_t kWaitNs = 2000000000ull;   // 2 s: the drain waits after an abort
 
 __device__ __forceinline__ int64_t mixed_offset(int32_t lin, int n, const int32_t *ext,
@@ -136,7 +152,7 @@ oz_split_kernel(const DPanel *__restrict__ panels, int32_t npanels,
         const DPanel &P = panels[p];
         const double *src = P.src ? B : A;
         uint8_t *base = slices + P.slice_off;
-        const int TR = P.src ? 64 : 128;             // rows per tile image (MMA N or M)
+        const int TR = P.tr;
         const int nkb = P.K_pad / kKbe;
         const bool contig = P.nk == 1 && P.kstr[0] == 1;
         for (int r0 = blockIdx.x * 32; r0 < P.rows_pad; r0 += gridDim.x * 32) {
@@ -156,6 +172,7 @@ oz_split_kernel(const DPanel *__restrict__ panels, int32_t npanels,
             mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
             int e = 0;
             if (mx > 0.0) frexp(mx, &e);            // mx = f * 2^e, f in [0.5, 1)
+            if (r >= P.rows_pad) continue;          // (after the shuffles of the warp's rows)
             if (c == 0) exps[P.exp_off + r] = e;
             const double up = ldexp(1.0, beta);
             for (int k0 = 4 * c; k0 < P.K_pad; k0 += 32) {
@@ -242,70 +259,48 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
         :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 
-// K-major shared-memory matrix descriptor without swizzle: 8-row x 16-byte
-// core matrices, the two k halves 128 bytes apart (leading byte offset),
-// 8-row groups 256 bytes apart (stride byte offset).
-__device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);          // start address
-    d |= (uint64_t)(128 >> 4) << 16;                  // leading byte offset
-    d |= (uint64_t)(256 >> 4) << 32;                  // stride byte offset
-    d |= (uint64_t)1 << 46;                           // descriptor version (sm_100)
-    return d;                                         // layout type 0: no swizzle
-}
+// K-major shared-memory matrix descriptor without swizzle (layout type 0):
+// 8-row x 16-byte core matrices, the two k halves 128 bytes apart (leading
+// byte offset), 8-row groups 256 bytes apart (stride byte offset), descriptor
+// version 1 (sm_100).  Low word: start address and leading offset in 16-byte
+// units; high word: stride offset and version.
+constexpr uint32_t kDescHi = (256u >> 4) | (1u << 14);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr >> 4) & 0x3FFF) | ((128u >> 4) << 16); }
 
 template<int KIND>
-__device__ __forceinline__ uint32_t instr_desc() {
+__device__ __forceinline__ uint32_t instr_desc(int n) {
     // D format: S32 for int8, F32 otherwise; A/B formats; K-major A and B;
-    // N = 64, M = 128.
+    // N = n (a multiple of 16, at most 256), M = 128.
     uint32_t c_fmt = KIND == kOzInt8 ? 2u : 1u;
     uint32_t ab_fmt = KIND == kOzInt8 ? 1u : (KIND == kOzBf16 ? 1u : 0u);
-    return (c_fmt << 4) | (ab_fmt << 7) | (ab_fmt << 10) | ((uint32_t)(kBN >> 3) << 17) |
+    return (c_fmt << 4) | (ab_fmt << 7) | (ab_fmt << 10) | ((uint32_t)(n >> 3) << 17) |
            ((uint32_t)(kBM >> 4) << 24);
 }
 
+// D (+)= A B^T; x and y are the low words of the operands' descriptors (the
+// high word is the same for every tile: kDescHi).  Formed by 32-bit adds from
+// one word per stage and with the instruction descriptors ready, an MMA costs
+// the issuing thread less than its run time; descriptors and piece widths
+// worked out per MMA cost it 260 clocks each (BF16 x 4, 6 MMAs of 112-224
+// columns per k block: 4.9 ms against 1.7 of products).
 template<int KIND>
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                     uint32_t accumulate) {
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint32_t x, uint32_t y, uint32_t idesc, uint32_t accumulate) {
     if (KIND == kOzInt8) {
-        asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                     "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p; }"
-                     :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        asm volatile("{ .reg .pred p; .reg .b64 a, b; mov.b64 a, {%1, %5}; mov.b64 b, {%2, %5};\n"
+                     "setp.ne.b32 p, %4, 0;\n"
+                     "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %3, p; }"
+                     :: "r"(tmem_d), "r"(x), "r"(y), "r"(idesc), "r"(accumulate), "n"(kDescHi) : "memory");
     } else if (KIND == kOzBf16) {
-        asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
-                     :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        asm volatile("{ .reg .pred p; .reg .b64 a, b; mov.b64 a, {%1, %5}; mov.b64 b, {%2, %5};\n"
+                     "setp.ne.b32 p, %4, 0;\n"
+                     "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p; }"
+                     :: "r"(tmem_d), "r"(x), "r"(y), "r"(idesc), "r"(accumulate), "n"(kDescHi) : "memory");
     } else {
-        asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                     "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p; }"
-                     :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        asm volatile("{ .reg .pred p; .reg .b64 a, b; mov.b64 a, {%1, %5}; mov.b64 b, {%2, %5};\n"
+                     "setp.ne.b32 p, %4, 0;\n"
+                     "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, p; }"
+                     :: "r"(tmem_d), "r"(x), "r"(y), "r"(idesc), "r"(accumulate), "n"(kDescHi) : "memory");
     }
-}
-
-// Same product with the A operand read from tensor memory (a_tmem).
-template<int KIND>
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    if (KIND == kOzInt8) {
-        asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                     "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p; }"
-                     :: "r"(tmem_d), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-    } else if (KIND == kOzBf16) {
-        asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                     "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }"
-                     :: "r"(tmem_d), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-    } else {
-        asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                     "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p; }"
-                     :: "r"(tmem_d), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-    }
-}
-
-// Shared -> tensor memory copy of one 128-row x 32-byte operand tile (row r
-// to TMEM lane r, 8 columns).  Executes in issue order with the MMAs of the
-// same thread, so a single A buffer can be refilled every k step.
-__device__ __forceinline__ void tmem_cp_128x256b(uint32_t taddr, uint64_t sdesc) {
-    asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" :: "r"(taddr), "l"(sdesc) : "memory");
 }
 
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
@@ -325,6 +320,49 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 
 // ---------------------------------------------------------------- slice products
 
+// 2^e f (|e| < 2044), by two normal powers of two: a test for one that fits,
+// with ldexp for the others, cost the epilogue 9,400 clocks per drain of
+// 128 x 112 elements.
+__device__ __forceinline__ double scale_exp(double f, int e) {
+    const int e1 = e >> 1, e2 = e - e1;
+    return (f * __hiloint2double((e1 + 1023) << 20, 0)) * __hiloint2double((e2 + 1023) << 20, 0);
+}
+
+// sum_l 2^(-beta l) acc_l of column j, acc_l the integer level sums v[l][j].
+// The levels are joined as integers, kGroup at a time, and only the groups
+// become doubles: with one FP32 -> FP64 conversion and one FMA per level the
+// epilogue took 34,000 clocks per drain of 57,000 sums, and takes 6,000 now.  FP32 sums (at most
+// (l + 1) / S 2^24 in magnitude, so two neighbours fit 32 bits: 2^beta (S - 1) /
+// S 2^24 + 2^24 < 2^31) are joined in fours, |.| < 2^46; INT32 sums in threes,
+// |.| < 2^46.  Every step is exact up to the final rounding.
+template<int KIND, int S>
+__device__ __forceinline__ double level_sum(const uint32_t (&v)[S][8], int j) {
+    constexpr int kBeta = KIND == kOzE4m3 ? 5 : 7;
+    constexpr int kGroup = KIND == kOzInt8 ? 3 : 4;
+    auto level = [&](int l) { return KIND == kOzInt8 ? (int)v[l][j] : __float2int_rn(__uint_as_float(v[l][j])); };
+    double sum = 0.0;
+#pragma unroll
+    for (int l0 = (S - 1) / kGroup * kGroup; l0 >= 0; l0 -= kGroup) {
+        const int l1 = l0 + kGroup < S ? l0 + kGroup : S;      // levels l0 .. l1 - 1
+        long long g;
+        if (KIND == kOzInt8) {
+            g = level(l0);
+#pragma unroll
+            for (int l = l0 + 1; l < l1; l++) g = (g << kBeta) + level(l);
+        } else if (l1 - l0 == 1) {
+            g = level(l0);
+        } else {
+            g = level(l0) * (1 << kBeta) + level(l0 + 1);
+            if (l1 - l0 == 3) g = g * (1 << kBeta) + level(l0 + 2);
+            if (l1 - l0 == 4) g = g * (1 << (2 * kBeta)) + (level(l0 + 2) * (1 << kBeta) + level(l0 + 3));
+        }
+        // int64 -> double by bits (|g| < 2^51)
+        const double d = __longlong_as_double(g + 0x4338000000000000ll) - 6755399441055744.0;
+        sum = fma(d, 1.0 / (double)(1ll << (kBeta * (l1 - 1))), sum);
+    }
+    return sum;
+}
+
 // SCATTER: each finished tile row goes, by atomic adds into a zeroed
 // result, to the destinations dests[drange[cblk]] of its C block (blocks of
 // another tensor with their own index mappings and scales: the terms of a
@@ -333,21 +371,14 @@ template<int KIND, int S, bool SCATTER = false>
 __global__ void __launch_bounds__(kThreads, 1)
 oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ slices,
                const DOzTask *__restrict__ tasks, const DCBlock *__restrict__ cblks,
-               const DItem *__restrict__ items, int32_t nitems, const int32_t *__restrict__ exps,
-               double *__restrict__ Cp, int32_t add, int32_t stages, int32_t chunk_kb,
-               int32_t beta0, int32_t beta, int32_t kbe, int32_t *err, uint64_t wait_ns,
+               const DOzItem *__restrict__ items, int32_t nitems, const int32_t *__restrict__ exps,
+               double *__restrict__ Cp, int32_t add, int32_t swap, int32_t stages, int32_t stage_bytes, int32_t kps,
+               int32_t chunk_kb, int32_t beta0, int32_t kbe, int32_t *err, uint64_t wait_ns,
                const int2 *__restrict__ drange = nullptr, const DCBlock *__restrict__ dests = nullptr) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
-    // 1024-byte aligned stage buffers: [stage][A slices | B slices]
+    // 1024-byte aligned stage buffers of kps k blocks: [stage][M-side slices | N-side slices]
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    constexpr int kStageBytes = S * (kATile + kBTile);
-    // A operand from tensor memory (tcgen05.cp of the A slices once per k
-    // step, products reading only B from shared memory) is supported when the
-    // accumulators leave room for it, but measured slower than reading both
-    // operands from shared memory on the ladder workloads (35.1 vs 39.4
-    // effective TFLOP/s at S = 7), so it is off.
-    constexpr bool kATmem = false && (S * kBN + S * 8 <= 512);
-    constexpr int kACol = S * kBN;
+    constexpr int kHalf = oz_max_nt(S) / 2;         // columns per epilogue thread, at most
     __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], accf_bar, acce_bar, drain_bar;
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_s;
@@ -356,7 +387,7 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
     if (threadIdx.x == 0) {
         for (int i = 0; i < stages; i++) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
         mbar_init(&accf_bar, 1);
-        mbar_init(&acce_bar, 4);
+        mbar_init(&acce_bar, kEpiWarps);
         mbar_init(&drain_bar, 1);
         abort_s = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -372,7 +403,7 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
     const uint32_t tmem = tmem_base_s;
     const uint32_t smem0 = smem_u32(smem);
 
-    if (warp == 4) {
+    if (warp == kEpiWarps) {
         // ------------------------------------------------ bulk-copy producer (1-D cp.async.bulk)
         if (lane == 0) {
             int st = 0;
@@ -381,22 +412,23 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
             int armed_parity[kMaxStages];
             for (int i = 0; i < kMaxStages; i++) armed_parity[i] = -1;
             for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
-                const DItem item = items[it];
+                const DOzItem item = items[it];
                 const DCBlock &cb = cblks[item.cblk];
+                const int ytile = item.nt * kRowBytes;
                 for (int ti = cb.t_begin; ti < cb.t_end && ok; ti++) {
                     const DOzTask t = tasks[ti];
-                    const int nkb = panels[t.pa].K_pad / kbe;
+                    const int nkb = panels[t.px].K_pad / kbe;
                     // tile images of this (row tile, k block): all S slices contiguous
-                    const uint8_t *ga = slices + panels[t.pa].slice_off + (int64_t)(item.m0 / kBM) * nkb * S * kATile;
-                    const uint8_t *gb = slices + panels[t.pb].slice_off + (int64_t)(item.n0 / kBN) * nkb * S * kBTile;
-                    for (int kb = 0; kb < nkb; kb++) {
+                    const uint8_t *gx = slices + panels[t.px].slice_off + (int64_t)(item.x0 / kBM) * nkb * S * kXTile;
+                    const uint8_t *gy = slices + panels[t.py].slice_off + (int64_t)(item.y0 / item.nt) * nkb * S * ytile;
+                    for (int kb = 0; kb < nkb; kb += kps) {
                         if (!mbar_wait(&empty_bar[st], ph ^ 1, &abort_s, wait_ns)) { ok = false; break; }
-                        const uint32_t sa = smem0 + st * kStageBytes;
-                        const uint32_t sb = sa + S * kATile;
+                        const uint32_t sx = smem0 + st * stage_bytes;
                         const uint32_t fb = smem_u32(&full_bar[st]);
-                        mbar_expect_tx(&full_bar[st], (uint32_t)kStageBytes);
-                        bulk_load(sa, ga + (int64_t)kb * S * kATile, S * kATile, fb);
-                        bulk_load(sb, gb + (int64_t)kb * S * kBTile, S * kBTile, fb);
+                        const uint32_t slabs = (uint32_t)(min(kps, nkb - kb) * S);
+                        mbar_expect_tx(&full_bar[st], slabs * (uint32_t)(kXTile + ytile));
+                        bulk_load(sx, gx + (int64_t)kb * S * kXTile, slabs * kXTile, fb);
+                        bulk_load(sx + kps * S * kXTile, gy + (int64_t)kb * S * ytile, slabs * (uint32_t)ytile, fb);
                         armed_parity[st] = (int)ph;
                         if (++st == stages) { st = 0; ph ^= 1; }
                     }
@@ -413,19 +445,29 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
             for (int i = 0; i < stages; i++)
                 if (armed_parity[i] >= 0) (void)mbar_wait(&full_bar[i], (uint32_t)armed_parity[i], &never, kWaitNs);
         }
-    } else if (warp == 5) {
+    } else if (warp == kEpiWarps + 1) {
         // ------------------------------------------------ MMA issuer
         if (lane == 0) {
-            const uint32_t idesc = instr_desc<KIND>();
             int st = 0;
             uint32_t ph = 0, accph = 0;
             int ndrain = 0;
             bool ok = true;
             for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
-                const DItem item = items[it];
+                const DOzItem item = items[it];
                 const DCBlock &cb = cblks[item.cblk];
+                // per M-side slice: its columns in one piece, or in two (the
+                // first of w columns) where the widest tile needs them
+                uint32_t id0[S], id1[S];
+                int w[S];
+#pragma unroll
+                for (int sa = 0; sa < S; sa++) {
+                    const int cols = (S - sa) * item.nt;
+                    w[sa] = two_pieces<S>(sa) ? (cols / 2 + 15) / 16 * 16 : cols;
+                    id0[sa] = instr_desc<KIND>(w[sa]);
+                    id1[sa] = instr_desc<KIND>(cols - w[sa]);
+                }
                 for (int ti = cb.t_begin; ti < cb.t_end && ok; ti++) {
-                    const int nkb = panels[tasks[ti].pa].K_pad / kbe;
+                    const int nkb = panels[tasks[ti].px].K_pad / kbe;
                     for (int kb0 = 0; kb0 < nkb && ok; kb0 += chunk_kb) {
                         // the accumulators are free once the previous drain was read
                         if (ndrain > 0) {
@@ -434,37 +476,26 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
                         }
                         tc_fence_after();
                         const int kb1 = min(nkb, kb0 + chunk_kb);
-                        for (int kb = kb0; kb < kb1; kb++) {
+                        uint32_t acc = 0;
+                        for (int kb = kb0; kb < kb1; kb += kps) {
                             if (!mbar_wait(&full_bar[st], ph, &abort_s, wait_ns)) { ok = false; break; }
                             tc_fence_after();
-                            const uint32_t a0 = smem0 + st * kStageBytes;
-                            const uint32_t b0 = a0 + S * kATile;
-                            const uint64_t da = smem_desc_kmajor(a0), db = smem_desc_kmajor(b0);
-                            const uint32_t first = kb == kb0 ? 0u : 1u;
-                            if (kATmem) {
-                                // A slices into tensor memory once per k step; the
-                                // products then read only B from shared memory.
+                            const int nsub = min(kps, kb1 - kb);
+                            uint32_t dx = desc_lo(smem0 + st * stage_bytes);
+                            uint32_t dy = dx + (uint32_t)((kps * S * kXTile) >> 4);
+                            for (int j = 0; j < nsub; j++) {
 #pragma unroll
-                                for (int sa = 0; sa < S; sa++)
-                                    tmem_cp_128x256b(tmem + (uint32_t)(kACol + sa * 8),
-                                                     da + (uint64_t)((sa * kATile) >> 4));
-                            }
-#pragma unroll
-                            for (int l = 0; l < S; l++) {
-#pragma unroll
-                                for (int sa = 0; sa <= l; sa++) {
-                                    const int sb = l - sa;
-                                    // descriptor start addresses advance in 16-byte units
-                                    if (kATmem)
-                                        umma_ts<KIND>(tmem + (uint32_t)(l * kBN), tmem + (uint32_t)(kACol + sa * 8),
-                                                      db + (uint64_t)((sb * kBTile) >> 4), idesc,
-                                                      sa == 0 ? first : 1u);
-                                    else
-                                        umma<KIND>(tmem + (uint32_t)(l * kBN),
-                                                   da + (uint64_t)((sa * kATile) >> 4),
-                                                   db + (uint64_t)((sb * kBTile) >> 4), idesc,
-                                                   sa == 0 ? first : 1u);
+                                for (int sa = 0; sa < S; sa++) {
+                                    const uint32_t xa = dx + (uint32_t)((sa * kXTile) >> 4);
+                                    const uint32_t da = tmem + (uint32_t)(sa * item.nt);
+                                    umma<KIND>(da, xa, dy, id0[sa], sa == 0 ? acc : 1u);
+                                    if (two_pieces<S>(sa))
+                                        umma<KIND>(da + (uint32_t)w[sa], xa, dy + (uint32_t)((w[sa] * kRowBytes) >> 4),
+                                                   id1[sa], sa == 0 ? acc : 1u);
                                 }
+                                acc = 1;
+                                dx += (uint32_t)((S * kXTile) >> 4);
+                                dy += (uint32_t)((S * item.nt * kRowBytes) >> 4);
                             }
                             umma_commit(&empty_bar[st]);       // frees the stage when these MMAs finish
                             if (++st == stages) { st = 0; ph ^= 1; }
@@ -484,29 +515,30 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
             }
         }
     } else {
-        // ------------------------------------------------ epilogue (warps 0-3)
-        const int row = warp * 32 + lane;                 // TMEM lane == tile row
-        const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
+        // ------------------------------------------------ epilogue (warps 0-7)
+        // warp w reads TMEM lanes 32 (w % 4) .. + 31 and the first or second
+        // half of the tile's columns
+        const int row = (warp & 3) * 32 + lane;           // TMEM lane == tile row
+        const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         uint32_t accph = 0;
         bool ok = true;
-        double lw[S];                                     // 2^(-beta * l)
-        lw[0] = 1.0;
-#pragma unroll
-        for (int l = 1; l < S; l++) lw[l] = ldexp(lw[l - 1], -beta);
         for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
-            const DItem item = items[it];
+            const DOzItem item = items[it];
             const DCBlock &cb = cblks[item.cblk];
-            double acc[kBN];
+            const int hc = item.nt >> 1, c0 = (warp >> 2) * hc;    // nt is a multiple of 16
+            double acc[kHalf];
 #pragma unroll
-            for (int j = 0; j < kBN; j++) acc[j] = 0.0;
-            const int m = item.m0 + row;
+            for (int j = 0; j < kHalf; j++) acc[j] = 0.0;
+            const int x = item.x0 + row;
             for (int ti = cb.t_begin; ti < cb.t_end && ok; ti++) {
                 const DOzTask t = tasks[ti];
-                const DPanel &pa = panels[t.pa];
-                const DPanel &pb = panels[t.pb];
-                const int nkb = pa.K_pad / kbe;
-                const double f = ldexp(t.coeff, exps[pa.exp_off + m] - 2 * beta0);
-                const int32_t *eb = exps + pb.exp_off + item.n0;
+                const DPanel &px = panels[t.px];
+                const DPanel &py = panels[t.py];
+                const int nkb = px.K_pad / kbe;
+                const double f = ldexp(t.coeff, exps[px.exp_off + x] - 2 * beta0);
+                // the columns' exponents, one or two per lane
+                const int32_t *ey = exps + py.exp_off + item.y0 + c0;
+                const int e_lo = lane < hc ? ey[lane] : 0, e_hi = kHalf > 32 && lane + 32 < hc ? ey[lane + 32] : 0;
                 for (int kb0 = 0; kb0 < nkb; kb0 += chunk_kb) {
                     // warp-uniform outcome: tcgen05.ld below is .sync.aligned
                     ok = __all_sync(0xffffffffu, mbar_wait(&accf_bar, accph, &abort_s, wait_ns));
@@ -514,21 +546,16 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
                     accph ^= 1;
                     tc_fence_after();
 #pragma unroll
-                    for (int c = 0; c < kBN / 8; c++) {
+                    for (int c = 0; c < kHalf / 8; c++) {
+                        if (c * 8 >= hc) continue;        // uniform over the CTA
                         uint32_t v[S][8];
 #pragma unroll
-                        for (int l = 0; l < S; l++) tmem_ld8(lane_base + (uint32_t)(l * kBN + c * 8), v[l]);
+                        for (int l = 0; l < S; l++) tmem_ld8(lane_base + (uint32_t)(l * item.nt + c0 + c * 8), v[l]);
                         tmem_wait_ld();
 #pragma unroll
                         for (int j = 0; j < 8; j++) {
-                            double sum = 0.0;
-#pragma unroll
-                            for (int l = S - 1; l >= 0; l--) {
-                                const double x = KIND == kOzInt8 ? (double)(int32_t)v[l][j]
-                                                                 : (double)__uint_as_float(v[l][j]);
-                                sum += lw[l] * x;
-                            }
-                            acc[c * 8 + j] += ldexp(f, eb[c * 8 + j]) * sum;
+                            const int e = __shfl_sync(0xffffffffu, c * 8 + j < 32 ? e_lo : e_hi, (c * 8 + j) & 31);
+                            acc[c * 8 + j] += scale_exp(f, e) * level_sum<KIND, S>(v, j);
                         }
                     }
                     tc_fence_before();
@@ -537,34 +564,40 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
                 }
             }
             if (!ok) break;
-            // FP64 write of the finished tile row
-            if constexpr (SCATTER) {
-                if (m < cb.M) {
+            // FP64 write of the finished tile row: a C row, or with the sides
+            // swapped a C column
+            const int xe = swap ? cb.N : cb.M, ye = swap ? cb.M : cb.N;
+            auto offset = [&](const DCBlock &b, bool xside, int i) {
+                return xside != (swap != 0) ? mixed_offset(i, b.nm, b.mext, b.mc_str)
+                                            : mixed_offset(i, b.nn, b.next, b.nc_str);
+            };
+            if (x < xe) {
+                if constexpr (SCATTER) {
                     const int2 dr = drange[item.cblk];
                     for (int d = dr.x; d < dr.y; d++) {
                         const DCBlock &db = dests[d];
-                        const int64_t drow = db.c_off + mixed_offset(m, db.nm, db.mext, db.mc_str);
+                        const int64_t drow = db.c_off + offset(db, true, x);
 #pragma unroll
-                        for (int j = 0; j < kBN; j++) {
-                            const int n = item.n0 + j;
-                            if (n < cb.N)
-                                atomicAdd(Cp + drow + mixed_offset(n, db.nn, db.next, db.nc_str), db.scale * acc[j]);
+                        for (int j = 0; j < kHalf; j++) {
+                            const int y = item.y0 + c0 + j;
+                            if (j < hc && y < ye) atomicAdd(Cp + drow + offset(db, false, y), db.scale * acc[j]);
+                        }
+                    }
+                } else {
+                    const int64_t orow = cb.c_off + offset(cb, true, x);
+#pragma unroll
+                    for (int j = 0; j < kHalf; j++) {
+                        const int y = item.y0 + c0 + j;
+                        if (j < hc && y < ye) {
+                            double *dst = Cp + orow + offset(cb, false, y);
+                            const double val = cb.scale * acc[j];
+                            if (add) *dst += val;
+                            else *dst = val;
                         }
                     }
                 }
-            } else if (m < cb.M) {
-                const int64_t orow = cb.c_off + mixed_offset(m, cb.nm, cb.mext, cb.mc_str);
-#pragma unroll
-                for (int j = 0; j < kBN; j++) {
-                    const int n = item.n0 + j;
-                    if (n < cb.N) {
-                        double *dst = Cp + orow + mixed_offset(n, cb.nn, cb.next, cb.nc_str);
-                        const double v = cb.scale * acc[j];
-                        if (add) *dst += v;
-                        else *dst = v;
-                    }
-                }
             }
+            __syncwarp();
         }
         if (!ok) { abort_s = 1; atomicExch(err, 7); }
     }
@@ -579,16 +612,35 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
 
 int g_nsm = 0;
 
+// What one slice-products launch takes besides its template arguments.
+struct OzGemmArgs {
+    const DPanel *panels;
+    const uint8_t *slices;
+    const DOzTask *tasks;
+    const DCBlock *cblks;
+    const DOzItem *items;
+    int32_t nitems;
+    const int32_t *exps;
+    double *c;
+    int32_t add, swap, chunk_kb, max_nt;
+    int32_t *err;
+    uint64_t wait_ns;
+    cudaStream_t s;
+    const int2 *drange;
+    const DCBlock *dests;
+};
+
 template<int KIND, int S, bool SCATTER = false>
-cudaError_t launch_gemm_s(const DPanel *panels, const uint8_t *slices, const DOzTask *tasks, const DCBlock *cblks,
-                          const DItem *items, int32_t nitems, const int32_t *exps, double *c, int32_t add,
-                          int32_t chunk_kb, int32_t *err, uint64_t wait_ns, cudaStream_t s,
-                          const int2 *drange = nullptr, const DCBlock *dests = nullptr) {
+cudaError_t launch_gemm_s(const OzGemmArgs &a) {
     int beta0, beta, esz, kbe;
     int64_t mp;
     oz_kind_params(KIND, &beta0, &beta, &esz, &kbe, &mp);
-    constexpr int stage_bytes = S * (kATile + kBTile);
-    int stages = (200 * 1024) / stage_bytes;
+    // two k blocks per stage while three such stages fit (half the barriers and
+    // copies per product); a chunk is then a whole number of stages
+    int stage_bytes = S * (kXTile + a.max_nt * kRowBytes), kps = 1;
+    if (a.chunk_kb >= 2 && 3 * 2 * stage_bytes <= kStageSmem) { kps = 2; stage_bytes *= 2; }
+    const int chunk_kb = a.chunk_kb / kps * kps;
+    int stages = kStageSmem / stage_bytes;
     if (stages > kMaxStages) stages = kMaxStages;
     if (stages < 2) return cudaErrorInvalidValue;
     // At least 120 KB so that a second CTA never shares the SM: each CTA
@@ -603,27 +655,52 @@ cudaError_t launch_gemm_s(const DPanel *panels, const uint8_t *slices, const DOz
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&g_nsm, cudaDevAttrMultiProcessorCount, dev);
     }
-    int grid = nitems < g_nsm ? nitems : g_nsm;
+    int grid = a.nitems < g_nsm ? a.nitems : g_nsm;
     if (grid < 1) return cudaSuccess;
-    oz_gemm_kernel<KIND, S, SCATTER><<<grid, kThreads, smem, s>>>(panels, slices, tasks, cblks, items, nitems, exps,
-                                                                 c, add, stages, chunk_kb, beta0, beta, kbe, err,
-                                                                 wait_ns, drange, dests);
+    oz_gemm_kernel<KIND, S, SCATTER><<<grid, kThreads, smem, a.s>>>(
+        a.panels, a.slices, a.tasks, a.cblks, a.items, a.nitems, a.exps, a.c, SCATTER ? 0 : a.add, a.swap, stages,
+        stage_bytes, kps, chunk_kb, beta0, kbe, a.err, a.wait_ns, a.drange, a.dests);
     return cudaGetLastError();
 }
 
 template<int KIND>
-cudaError_t launch_gemm_k(int S, const DPanel *panels, const uint8_t *slices, const DOzTask *tasks,
-                          const DCBlock *cblks, const DItem *items, int32_t nitems, const int32_t *exps, double *c,
-                          int32_t add, int32_t chunk_kb, int32_t *err, uint64_t wait_ns, cudaStream_t s) {
+cudaError_t launch_gemm_k(int S, const OzGemmArgs &a) {
     switch (S) {
-#define CASE_S(n) case n: return launch_gemm_s<KIND, n>(panels, slices, tasks, cblks, items, nitems, exps, c, add, chunk_kb, err, wait_ns, s);
+#define CASE_S(n) case n: return launch_gemm_s<KIND, n>(a);
     CASE_S(1) CASE_S(2) CASE_S(3) CASE_S(4) CASE_S(5) CASE_S(6) CASE_S(7) CASE_S(8)
 #undef CASE_S
     default: return cudaErrorInvalidValue;
     }
 }
 
+// Clocks per k block of one 128 x nt tile: its S(S+1)/2 products at nt / 2
+// clocks each, or its operand images from L2 at kL2Bytes per clock and SM
+// (about 11.6 TB/s over the chip), whichever is longer.  The rule takes nt = 112
+// for 400 rows and 4 slices (4 tiles, 89 % of their columns used), 64 for 7
+// and 8.  Ladder o=40 v=240, BF16 x 4: products 8.58 ms with 128 x 64 tiles and
+// one MMA per slice pair, 3.38 now; o=30 v=150, FP8 x 8: 0.99 to 0.60 ms.
+constexpr double kL2Bytes = 42.0;
+double oz_tile_clocks(int nt, int S) {
+    const double mma = 0.25 * S * (S + 1) * nt, copy = S * (kXTile + nt * kRowBytes) / kL2Bytes;
+    return mma > copy ? mma : copy;
+}
+
 }  // namespace
+
+int32_t oz_tile_width(int64_t rows, int S) {
+    int32_t best = 16;
+    double cost = 1e300;
+    for (int32_t nt = 16; nt <= oz_max_nt(S); nt += 16) {
+        const double c = (double)((rows + nt - 1) / nt) * oz_tile_clocks(nt, S);
+        if (c <= cost) { cost = c; best = nt; }
+    }
+    return best;
+}
+
+double oz_product_cost(int64_t x, int64_t y, int S) {
+    const int32_t nt = oz_tile_width(y, S);
+    return (double)((x + kBM - 1) / kBM) * (double)((y + nt - 1) / nt) * oz_tile_clocks(nt, S);
+}
 
 cudaError_t launch_oz_split(int kind, const DPanel *panels, int32_t npanels, int32_t max_rows_pad,
                             const double *a, const double *b, uint8_t *slices, int32_t *exps,
@@ -643,31 +720,22 @@ cudaError_t launch_oz_split(int kind, const DPanel *panels, int32_t npanels, int
 }
 
 cudaError_t launch_oz_gemm(int kind, const DPanel *panels, const uint8_t *slices, const DOzTask *tasks,
-                           const DCBlock *cblks, const DItem *items, int32_t nitems, const int32_t *exps,
-                           double *c, int32_t add, int32_t S, int32_t chunk_kb, int32_t *err,
-                           uint64_t wait_ns, cudaStream_t s, const int2 *drange, const DCBlock *dests) {
-    if (S < 1 || S > 8) return cudaErrorInvalidValue;
+                           const DCBlock *cblks, const DOzItem *items, int32_t nitems, const int32_t *exps,
+                           double *c, int32_t add, int32_t S, int32_t swap, int32_t chunk_kb, int32_t max_nt,
+                           int32_t *err, uint64_t wait_ns, cudaStream_t s, const int2 *drange, const DCBlock *dests) {
+    if (S < 1 || S > 8 || max_nt > oz_max_nt(S)) return cudaErrorInvalidValue;
+    const OzGemmArgs a{panels, slices, tasks, cblks, items, nitems, exps, c, add, swap, chunk_kb, max_nt,
+                       err, wait_ns, s, drange, dests};
     if (dests) {
         // the scattering form for each kind's default slice count only
-        if (kind == kOzInt8 && S == 7)
-            return launch_gemm_s<kOzInt8, 7, true>(panels, slices, tasks, cblks, items, nitems, exps, c, 0, chunk_kb,
-                                                   err, wait_ns, s, drange, dests);
-        if (kind == kOzBf16 && S == 7)
-            return launch_gemm_s<kOzBf16, 7, true>(panels, slices, tasks, cblks, items, nitems, exps, c, 0, chunk_kb,
-                                                   err, wait_ns, s, drange, dests);
-        if (kind == kOzE4m3 && S == 8)
-            return launch_gemm_s<kOzE4m3, 8, true>(panels, slices, tasks, cblks, items, nitems, exps, c, 0, chunk_kb,
-                                                   err, wait_ns, s, drange, dests);
+        if (kind == kOzInt8 && S == 7) return launch_gemm_s<kOzInt8, 7, true>(a);
+        if (kind == kOzBf16 && S == 7) return launch_gemm_s<kOzBf16, 7, true>(a);
+        if (kind == kOzE4m3 && S == 8) return launch_gemm_s<kOzE4m3, 8, true>(a);
         return cudaErrorNotSupported;
     }
-    if (kind == kOzInt8)
-        return launch_gemm_k<kOzInt8>(S, panels, slices, tasks, cblks, items, nitems, exps, c, add, chunk_kb, err,
-                                      wait_ns, s);
-    if (kind == kOzBf16)
-        return launch_gemm_k<kOzBf16>(S, panels, slices, tasks, cblks, items, nitems, exps, c, add, chunk_kb, err,
-                                      wait_ns, s);
-    return launch_gemm_k<kOzE4m3>(S, panels, slices, tasks, cblks, items, nitems, exps, c, add, chunk_kb, err,
-                                  wait_ns, s);
+    if (kind == kOzInt8) return launch_gemm_k<kOzInt8>(S, a);
+    if (kind == kOzBf16) return launch_gemm_k<kOzBf16>(S, a);
+    return launch_gemm_k<kOzE4m3>(S, a);
 }
 
 }  // namespace ltg
