@@ -195,9 +195,9 @@ struct SymExec {
 // Device arrays of the split-precision path for one (C tensor, coefficients,
 // mode, slice count).
 struct OzExec {
-    int kind = 0, S = 0, chunk_kb = 1, npanels = 0, max_rows_pad = 0, nitems = 0, swap = 0, max_nt = 16;
+    int kind = 0, S = 0, chunk_kb = 1, nunits = 0, nitems = 0, swap = 0, max_nt = 16;
     int64_t src_elems = 0, slice_bytes = 0;   // operand elements read, slice bytes written
-    DevBuf panels, slices, exps, tasks, cblks, items;
+    DevBuf panels, units, slices, exps, tasks, cblks, items;
     std::vector<std::pair<int64_t, int64_t>> zero_ranges;
     std::vector<int64_t> sched_slots;
 
@@ -862,17 +862,24 @@ OzExec *prepare_ozaki(ltg_plan *pl, ltg_bt *c, int mode, int S, double ka, doubl
     std::stable_sort(iv.begin(), iv.end(), [](const std::pair<double, DOzItem> &x, const std::pair<double, DOzItem> &y) { return x.first > y.first; });
     std::vector<DOzItem> items;
     for (auto &p : iv) items.push_back(p.second);
+    std::vector<int4> units;
     for (const DPanel &p : panels) {
-        ex->max_rows_pad = std::max(ex->max_rows_pad, p.rows_pad);
+        const int32_t ru = oz_split_unit_rows(p.K);
+        for (int32_t r0 = 0; r0 < p.rows; r0 += ru)
+            units.push_back(make_int4((int32_t)(&p - panels.data()), r0, std::min(ru, (p.rows - r0 + 7) / 8 * 8), 0));
         ex->src_elems += (int64_t)p.rows * p.K;
         ex->slice_bytes += (int64_t)S * p.rows_pad * p.K_pad * esz;
     }
 
     cudaStream_t s = pl->ctx->stream;
-    ex->npanels = (int)panels.size();
+    ex->nunits = (int)units.size();
     ex->nitems = (int)items.size();
     ex->slices.alloc(std::max<int64_t>(slice_bytes, 1024));
     ex->exps.alloc(std::max<int32_t>(exp_rows, 1) * sizeof(int32_t));
+    // the padding rows and k of the images stay zero
+    LTG_CUDA(cudaMemsetAsync(ex->slices.p, 0, std::max<int64_t>(slice_bytes, 1024), s));
+    LTG_CUDA(cudaMemsetAsync(ex->exps.p, 0, std::max<int32_t>(exp_rows, 1) * sizeof(int32_t), s));
+    upload_vec(ex->units, units, s);
     upload_vec(ex->panels, panels, s);
     upload_vec(ex->tasks, dt, s);
     upload_vec(ex->cblks, dc, s);
@@ -2852,7 +2859,7 @@ int ltg_contract2_symmetrized(ltg_plan *plan, ltg_bt *r, int32_t mode, int32_t n
         if (OzExec *ox = ex->oz) {
             report_device_wait(ctx);
             TimedLaunch t_split(ctx, LTG_KERNEL_OZ_SPLIT);
-            LTG_CUDA(launch_oz_split(ox->kind, ox->panels.as<DPanel>(), ox->npanels, ox->max_rows_pad,
+            LTG_CUDA(launch_oz_split(ox->kind, ox->panels.as<DPanel>(), ox->units.as<int4>(), ox->nunits,
                                      plan->a->arena.as<double>(), plan->b->arena.as<double>(),
                                      ox->slices.as<uint8_t>(), ox->exps.as<int32_t>(), ox->S, s));
             t_split.done();
@@ -3415,7 +3422,7 @@ int ltg_contract2(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nslices, doub
                 for (auto &r : ox->zero_ranges)
                     LTG_CUDA(cudaMemsetAsync(c->arena.as<double>() + r.first, 0, (r.second - r.first) * sizeof(double), s));
             TimedLaunch t_split(ctx, LTG_KERNEL_OZ_SPLIT);
-            LTG_CUDA(launch_oz_split(ox->kind, ox->panels.as<DPanel>(), ox->npanels, ox->max_rows_pad,
+            LTG_CUDA(launch_oz_split(ox->kind, ox->panels.as<DPanel>(), ox->units.as<int4>(), ox->nunits,
                                      plan->a->arena.as<double>(), plan->b->arena.as<double>(),
                                      ox->slices.as<uint8_t>(), ox->exps.as<int32_t>(), ox->S, s));
             t_split.done();

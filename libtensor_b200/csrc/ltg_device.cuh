@@ -320,8 +320,12 @@ int tile_cfg_bk(int cfg);
 
 // Split-precision contraction: FP64 -> slice tile images, then the tcgen05
 // grouped slice-product kernel with FP64 recombination.
-cudaError_t launch_oz_split(int kind, const DPanel *panels, int32_t npanels, int32_t max_rows_pad,
-    const double *a, const double *b, uint8_t *slices, int32_t *exps, int32_t S, cudaStream_t s);
+// Units (panel, first row, rows, unused): oz_split_unit_rows(K) rows of a
+// panel.  Writes rows < rows and k < K rounded up to 4; the padding of the
+// images and of the exponents must be zero before the first call.
+cudaError_t launch_oz_split(int kind, const DPanel *panels, const int4 *units, int32_t nunits, const double *a,
+    const double *b, uint8_t *slices, int32_t *exps, int32_t S, cudaStream_t s);
+int oz_split_unit_rows(int K);
 // With dests (one range drange[cblk] per C block), each C block's tile is
 // added atomically to its destinations (c zeroed before; add ignored); only
 // for each kind's default slice count (INT8 and BF16 7, FP8 8).

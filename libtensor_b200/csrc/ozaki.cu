@@ -89,34 +89,32 @@ __device__ __forceinline__ int64_t mixed_offset(int32_t lin, int n, const int32_
 
 // ---------------------------------------------------------------- split
 
-// Four consecutive slice values packed for one store.
+// Four consecutive integer slice values packed for one store.  Integers become
+// floats by bits (1.5 * 2^23 + i, exact); BF16 is then the float's high half
+// (at most 7 significant bits), E4M3 one conversion per pair.
+__device__ __forceinline__ float small_float(int i) { return __int_as_float(0x4B400000 + i) - 12582912.0f; }
+
 template<int KIND> struct Pack4;
 template<> struct Pack4<kOzInt8> {
     typedef uint32_t T;
-    __device__ static T pack(const double *v) {
-        return (uint32_t)(uint8_t)(int8_t)(int)v[0] | ((uint32_t)(uint8_t)(int8_t)(int)v[1] << 8) |
-               ((uint32_t)(uint8_t)(int8_t)(int)v[2] << 16) | ((uint32_t)(uint8_t)(int8_t)(int)v[3] << 24);
+    __device__ __forceinline__ static T pack(const int *v) {
+        return __byte_perm(__byte_perm(v[0], v[1], 0x0040), __byte_perm(v[2], v[3], 0x0040), 0x5410);
     }
 };
 template<> struct Pack4<kOzE4m3> {
     typedef uint32_t T;
-    __device__ static T pack(const double *v) {
-        uint32_t r = 0;
-        for (int i = 0; i < 4; i++) {
-            __nv_fp8_e4m3 q((float)v[i]);
-            r |= (uint32_t)q.__x << (8 * i);
-        }
-        return r;
+    __device__ __forceinline__ static T pack(const int *v) {
+        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(small_float(v[0]), small_float(v[1])), __NV_SATFINITE, __NV_E4M3);
+        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(small_float(v[2]), small_float(v[3])), __NV_SATFINITE, __NV_E4M3);
+        return lo | (hi << 16);
     }
 };
 template<> struct Pack4<kOzBf16> {
     typedef uint2 T;
-    __device__ static T pack(const double *v) {
-        __nv_bfloat16 b[4];
-        for (int i = 0; i < 4; i++) b[i] = __float2bfloat16_rn((float)v[i]);
+    __device__ __forceinline__ static T pack(const int *v) {
         uint2 r;
-        r.x = (uint32_t)__bfloat16_as_ushort(b[0]) | ((uint32_t)__bfloat16_as_ushort(b[1]) << 16);
-        r.y = (uint32_t)__bfloat16_as_ushort(b[2]) | ((uint32_t)__bfloat16_as_ushort(b[3]) << 16);
+        r.x = __byte_perm(__float_as_uint(small_float(v[0])), __float_as_uint(small_float(v[1])), 0x7632);
+        r.y = __byte_perm(__float_as_uint(small_float(v[2])), __float_as_uint(small_float(v[3])), 0x7632);
         return r;
     }
 };
@@ -134,66 +132,172 @@ __device__ __forceinline__ int64_t tile_image_offset(int r, int TR, int nkb, int
            (rr & 7) * 16 + (kb_byte & 15);
 }
 
-// 32 panel rows per CTA, 8 threads per row, 4 consecutive k per thread; two
-// passes over each row (largest magnitude, then the slices).  Contiguous
-// rows (one k sub-dimension of stride 1) skip the mixed-radix arithmetic.
-template<int KIND>
-__global__ void __launch_bounds__(256)
-oz_split_kernel(const DPanel *__restrict__ panels, int32_t npanels,
+// Units (panel, first row, rows, unused): a multiple of 8 rows of one panel,
+// all of its k, as core tiles of 8 rows x 16 k spread over the CTA's warps (lane l
+// takes row l / 4 and the four consecutive k of group l % 4, so that a warp
+// stores whole 128- or 256-byte runs of the tile images).  Two passes over the
+// unit: the rows' largest magnitudes, then the slices.  Bound by HBM: the
+// operand in once, S slices out.  So that the second pass reads L2, a unit of
+// long rows is 8 rows and two CTAs of 512 threads share an SM: 296 units of
+// 8 x 4096 doubles are 78 MB of the 126 MB L2; with 32-row units and eight
+// CTAs per SM both passes went to HBM.  Ladder o=40 v=240, BF16 x 4 (3.6 GB in,
+// 3.7 GB out): 2.37 ms to 1.82; o=30 v=150, FP8 x 8: 0.59 to 0.37 ms.
+// Slice s of t = x 2^(beta0 - e) is rint(t 2^(beta s)) of what the slices before
+// it left: t + 1.5 * 2^(52 - beta s) rounds to it and holds it in its low word;
+// what it leaves is exact.
+constexpr int kSplitThreads = 512;
+constexpr int kSplitWarps = kSplitThreads / 32;
+constexpr int kKoffMax = 4096;        // k offsets tabulated per unit
+constexpr int kUnitRowsMax = 256;
+
+template<int KIND, int S>
+__global__ void __launch_bounds__(kSplitThreads, 2)
+oz_split_kernel(const DPanel *__restrict__ panels, const int4 *__restrict__ units,
                 const double *__restrict__ A, const double *__restrict__ B,
-                uint8_t *__restrict__ slices, int32_t *__restrict__ exps, int32_t S,
-                int32_t beta0, int32_t beta) {
+                uint8_t *__restrict__ slices, int32_t *__restrict__ exps) {
     typedef typename Pack4<KIND>::T PT;
     constexpr int kEsz = KIND == kOzBf16 ? 2 : 1;
     constexpr int kKbe = 32 / kEsz;                  // elements per 32-byte k block
-    const int lr = threadIdx.x >> 3;                 // row within the CTA's 32 rows
-    const int c = threadIdx.x & 7;                   // 4-element chunk of a 32-element step
-    for (int p = blockIdx.y; p < npanels; p += gridDim.y) {
-        const DPanel &P = panels[p];
-        const double *src = P.src ? B : A;
-        uint8_t *base = slices + P.slice_off;
-        const int TR = P.tr;
-        const int nkb = P.K_pad / kKbe;
-        const bool contig = P.nk == 1 && P.kstr[0] == 1;
-        for (int r0 = blockIdx.x * 32; r0 < P.rows_pad; r0 += gridDim.x * 32) {
-            const int r = r0 + lr;
-            const bool valid = r < P.rows;
-            const double *row = src + (valid ? P.src_off + mixed_offset(r, P.nr, P.rext, P.rstr) : 0);
-            double mx = 0.0;
-            if (valid)
-                for (int k0 = 4 * c; k0 < P.K; k0 += 32)
+    constexpr int kBeta0 = KIND == kOzE4m3 ? 4 : 6, kBeta = kBeta0 + 1;
+    __shared__ int32_t koff[kKoffMax];
+    __shared__ int64_t roff[kUnitRowsMax];
+    __shared__ uint32_t rhi[kUnitRowsMax], rlo[kUnitRowsMax];   // largest high word of |x|, all low words or'ed
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lrow = lane >> 2, kq = lane & 3;
+    const int4 un = units[blockIdx.x];
+    const DPanel &P = panels[un.x];
+    const double *src = (P.src ? B : A) + P.src_off;
+    // k offsets: contiguous, tabulated, or computed per element
+    const int K = P.K, mode = P.nk == 0 || (P.nk == 1 && P.kstr[0] == 1) ? 0 : (K <= kKoffMax ? 1 : 2);
+    if (mode == 1)
+        for (int k = threadIdx.x; k < K; k += kSplitThreads) koff[k] = (int32_t)mixed_offset(k, P.nk, P.kext, P.kstr);
+    for (int i = threadIdx.x; i < un.z; i += kSplitThreads) {
+        rhi[i] = 0;
+        rlo[i] = 0;
+        roff[i] = un.y + i < P.rows ? mixed_offset(un.y + i, P.nr, P.rext, P.rstr) : -1;
+    }
+    __syncthreads();
+    const int nkt = (K + 15) >> 4, ngroups = un.z >> 3;
+    // This warp's core tiles: every kSplitWarps-th of the unit's, row group by
+    // row group.
+    struct Walk {
+        int rg, kt;
+        __device__ __forceinline__ void wrap(int nkt) { while (kt >= nkt) { kt -= nkt; rg++; } }
+    };
+    // four elements of this lane's row and k group in tile w (zero outside)
+    auto load4 = [&](const Walk &w, double *x) {
+        const int64_t ro = w.rg < ngroups ? roff[w.rg * 8 + lrow] : -1;
+        const int k0 = w.kt * 16 + kq * 4;
+        const double *row = src + ro;
+        if (ro >= 0 && mode == 0 && ((uintptr_t)row & 15) == 0 && k0 + 3 < K) {
+            const double2 a = *reinterpret_cast<const double2 *>(row + k0);
+            const double2 b = *reinterpret_cast<const double2 *>(row + k0 + 2);
+            x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+            return;
+        }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const int k = k0 + j;
-                        if (k < P.K) mx = fmax(mx, fabs(row[contig ? k : mixed_offset(k, P.nk, P.kext, P.kstr)]));
-                    }
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-            int e = 0;
-            if (mx > 0.0) frexp(mx, &e);            // mx = f * 2^e, f in [0.5, 1)
-            if (r >= P.rows_pad) continue;          // (after the shuffles of the warp's rows)
-            if (c == 0) exps[P.exp_off + r] = e;
-            const double up = ldexp(1.0, beta);
-            for (int k0 = 4 * c; k0 < P.K_pad; k0 += 32) {
-                double t[4], sg[4];
+        for (int j = 0; j < 4; j++) {
+            const int k = k0 + j;
+            x[j] = ro >= 0 && k < K ? row[mode == 0 ? k : mode == 1 ? koff[k] : mixed_offset(k, P.nk, P.kext, P.kstr)]
+                                    : 0.0;
+        }
+    };
+    {
+        // largest magnitudes, kept while the warp stays on its rows
+        uint32_t hi = 0, lo = 0;
+        int cur = -1;
+        auto flush = [&]() {
+            uint32_t h = hi, l = lo;
+            h = max(h, __shfl_xor_sync(0xffffffffu, h, 1));
+            h = max(h, __shfl_xor_sync(0xffffffffu, h, 2));
+            l |= __shfl_xor_sync(0xffffffffu, l, 1);
+            l |= __shfl_xor_sync(0xffffffffu, l, 2);
+            if (kq == 0) {
+                atomicMax(&rhi[cur * 8 + lrow], h);
+                atomicOr(&rlo[cur * 8 + lrow], l);
+            }
+            hi = lo = 0;
+        };
+        Walk w{0, warp};
+        w.wrap(nkt);
+        while (w.rg < ngroups) {
+            constexpr int kAhead = 4;                 // tiles loaded together
+            double x[kAhead][4];
+            Walk q[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                q[u] = w;
+                load4(w, x[u]);
+                w.kt += kSplitWarps;
+                w.wrap(nkt);
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                if (q[u].rg >= ngroups) break;        // uniform over the warp
+                if (q[u].rg != cur) {
+                    if (cur >= 0) flush();
+                    cur = q[u].rg;
+                }
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
-                    const int k = k0 + j;
-                    const double x = (valid && k < P.K) ? row[contig ? k : mixed_offset(k, P.nk, P.kext, P.kstr)] : 0.0;
-                    t[j] = ldexp(x, beta0 - e);     // |t| < 2^beta0, exact
-                }
-                const int kb = k0 / kKbe, kb_byte = (k0 % kKbe) * kEsz;
-                for (int s = 0; s < S; s++) {
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        sg[j] = rint(t[j]);
-                        t[j] = (t[j] - sg[j]) * up;   // exact (Sterbenz), power-of-two scale
-                    }
-                    *reinterpret_cast<PT *>(base + tile_image_offset(r, TR, nkb, kb, s, S, kb_byte)) =
-                        Pack4<KIND>::pack(sg);
+                    hi = max(hi, (uint32_t)__double2hiint(x[u][j]) & 0x7fffffffu);
+                    lo |= (uint32_t)__double2loint(x[u][j]);
                 }
             }
+        }
+        if (cur >= 0) flush();
+    }
+    __syncthreads();
+    const int TR = P.tr, nkb = P.K_pad / kKbe, sstep = TR * kRowBytes;
+    int cur = -1;
+    uint8_t *rowdst = nullptr;
+    double s1 = 1.0, s2 = 1.0;
+    bool one = true;
+    Walk w{0, warp};
+    w.wrap(nkt);
+    double nx[4];
+    load4(w, nx);
+    while (w.rg < ngroups) {
+        const Walk q = w;
+        double x[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[j] = nx[j];
+        w.kt += kSplitWarps;
+        w.wrap(nkt);
+        load4(w, nx);                                 // the next tile's, while this one is cut
+        const int i = q.rg * 8 + lrow, r = un.y + i, k0 = q.kt * 16 + kq * 4;
+        if (q.rg != cur) {
+            cur = q.rg;
+            // exponent of the row's largest element (|x| < 2^e): its high word
+            // has it, or, below 2^-1042, the highest low bit of the row
+            int e = 0;
+            if (rhi[i] | rlo[i]) frexp(__hiloint2double((int)rhi[i], (int)rlo[i]), &e);
+            if (r < P.rows && q.kt == 0 && kq == 0) exps[P.exp_off + r] = e;
+            // 2^(beta0 - e), as two finite factors where one would not do
+            const int sh = kBeta0 - e;
+            one = sh >= -1000 && sh <= 1000;
+            s1 = ldexp(1.0, one ? sh : sh / 2);
+            s2 = one ? 1.0 : ldexp(1.0, sh - sh / 2);
+            rowdst = slices + P.slice_off + tile_image_offset(r, TR, nkb, 0, 0, S, 0);
+        }
+        if (r >= P.rows || k0 >= K) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[j] *= s1;       // |x| < 2^beta0, exact
+        if (!one)
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[j] *= s2;
+        const int byte = (k0 % kKbe) * kEsz;
+        uint8_t *dst = rowdst + (int64_t)(k0 / kKbe) * S * sstep + (byte >> 4) * 128 + (byte & 15);
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            const double magic = 6755399441055744.0 / (double)(1ll << (kBeta * s));   // 1.5 * 2^(52 - beta s)
+            int v[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const double y = x[j] + magic;
+                v[j] = __double2loint(y);
+                x[j] -= y - magic;
+            }
+            *reinterpret_cast<PT *>(dst + s * sstep) = Pack4<KIND>::pack(v);
         }
     }
 }
@@ -702,20 +806,24 @@ double oz_product_cost(int64_t x, int64_t y, int S) {
     return (double)((x + kBM - 1) / kBM) * (double)((y + nt - 1) / nt) * oz_tile_clocks(nt, S);
 }
 
-cudaError_t launch_oz_split(int kind, const DPanel *panels, int32_t npanels, int32_t max_rows_pad,
-                            const double *a, const double *b, uint8_t *slices, int32_t *exps,
-                            int32_t S, cudaStream_t s) {
-    if (npanels <= 0) return cudaSuccess;
-    int beta0, beta, esz, kbe;
-    int64_t mp;
-    oz_kind_params(kind, &beta0, &beta, &esz, &kbe, &mp);
-    dim3 grid((max_rows_pad + 31) / 32, npanels < 65535 ? npanels : 65535);
-    if (kind == kOzInt8)
-        oz_split_kernel<kOzInt8><<<grid, 256, 0, s>>>(panels, npanels, a, b, slices, exps, S, beta0, beta);
-    else if (kind == kOzBf16)
-        oz_split_kernel<kOzBf16><<<grid, 256, 0, s>>>(panels, npanels, a, b, slices, exps, S, beta0, beta);
-    else
-        oz_split_kernel<kOzE4m3><<<grid, 256, 0, s>>>(panels, npanels, a, b, slices, exps, S, beta0, beta);
+int oz_split_unit_rows(int K) {
+    // about 64 core tiles (8 rows x 16 k) per unit of short rows, else 8 rows
+    const int nkt = (K + 15) / 16;
+    const int g = 64 / nkt;
+    return 8 * (g < 1 ? 1 : g > kUnitRowsMax / 8 ? kUnitRowsMax / 8 : g);
+}
+
+cudaError_t launch_oz_split(int kind, const DPanel *panels, const int4 *units, int32_t nunits, const double *a,
+                            const double *b, uint8_t *slices, int32_t *exps, int32_t S, cudaStream_t s) {
+    if (nunits <= 0) return cudaSuccess;
+    switch (kind * 16 + S) {
+#define CASE_KS(k, n) case k * 16 + n: oz_split_kernel<k, n><<<nunits, kSplitThreads, 0, s>>>(panels, units, a, b, slices, exps); break;
+#define CASE_K(k) CASE_KS(k, 1) CASE_KS(k, 2) CASE_KS(k, 3) CASE_KS(k, 4) CASE_KS(k, 5) CASE_KS(k, 6) CASE_KS(k, 7) CASE_KS(k, 8)
+    CASE_K(kOzInt8) CASE_K(kOzBf16) CASE_K(kOzE4m3)
+#undef CASE_K
+#undef CASE_KS
+    default: return cudaErrorInvalidValue;
+    }
     return cudaGetLastError();
 }
 
