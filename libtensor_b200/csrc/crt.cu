@@ -682,8 +682,8 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
                 const DCrtTask *__restrict__ tasks, const DCrtItem *__restrict__ items,
                 const int32_t *__restrict__ cta_items, uint8_t *__restrict__ out, const CrtParams cp,
                 int32_t stages, int32_t *err, uint64_t wait_ns) {
-    // this CTA's items: cta_items[j], j in [cta_items[b], cta_items[b + 1])
-    // (every role walks the same list)
+    // this CTA's work: pairs (item, moduli l0 | l1 << 8) at cta_items[j],
+    // j in [cta_items[b], cta_items[b + 1]) (every role walks the same list)
     const int j0 = cta_items[blockIdx.x], j1 = cta_items[blockIdx.x + 1];
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -719,11 +719,11 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
             bool ok = true;
             int armed[kMaxStages];
             for (int i = 0; i < kMaxStages; i++) armed[i] = -1;
-            for (int j = j0; j < j1 && ok; j++) {
-                const int it = cta_items[j];
-                const DCrtItem item = items[it];
+            for (int j = j0; j < j1 && ok; j += 2) {
+                const DCrtItem item = items[cta_items[j]];
+                const int l0 = cta_items[j + 1] & 255, l1 = cta_items[j + 1] >> 8;
                 const uint32_t ybytes = (uint32_t)item.nt * kKB;
-                for (int l = 0; l < L && ok; l++) {
+                for (int l = l0; l < l1 && ok; l++) {
                     for (int ti = item.t_begin; ti < item.t_end && ok; ti++) {
                         const DCrtTask t = tasks[ti];
                         const int nkb = t.nkb;
@@ -767,11 +767,11 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
             uint32_t uses[2] = {0, 0};               // fills of each accumulator slot so far
             int rr = 0;                              // slot of the next one-tile fill
             bool ok = true;
-            for (int j = j0; j < j1 && ok; j++) {
-                const int it = cta_items[j];
-                const DCrtItem item = items[it];
+            for (int j = j0; j < j1 && ok; j += 2) {
+                const DCrtItem item = items[cta_items[j]];
+                const int l0 = cta_items[j + 1] & 255, l1 = cta_items[j + 1] >> 8;
                 const uint32_t idesc = instr_desc_i8(item.nt);
-                for (int l = 0; l < L && ok; l++) {
+                for (int l = l0; l < l1 && ok; l++) {
                     // a two-tile fill takes both slots, a one-tile fill slot rr
                     const int s0 = item.nx == 2 ? 0 : rr;
                     // the epilogue has read the slots' previous fills
@@ -828,10 +828,10 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
         uint32_t uses[2] = {0, 0};                                // same slot sequence as the MMA warp
         int rr = 0;
         bool ok = true;
-        for (int j = j0; j < j1 && ok; j++) {
-            const int it = cta_items[j];
-            const DCrtItem item = items[it];
-            for (int l = 0; l < L; l++) {
+        for (int j = j0; j < j1 && ok; j += 2) {
+            const DCrtItem item = items[cta_items[j]];
+            const int l0 = cta_items[j + 1] & 255, l1 = cta_items[j + 1] >> 8;
+            for (int l = l0; l < l1; l++) {
                 const int s0 = item.nx == 2 ? 0 : rr;
                 ok = __all_sync(0xffffffffu, mbar_wait(&accf_bar[s0], uses[s0] & 1, &abort_s, wait_ns));
                 if (ok && item.nx == 2) ok = __all_sync(0xffffffffu, mbar_wait(&accf_bar[1], uses[1] & 1, &abort_s, wait_ns));
@@ -1077,9 +1077,10 @@ cudaError_t launch_crt_exponents(const DCrtPanel *panels, const int4 *units, int
     return cudaGetLastError();
 }
 
-cudaError_t launch_crt_fill(int32_t nx, int32_t ny, int32_t *ex, int32_t *ey, cudaStream_t s) {
-    crt_fill_kernel<<<64, 256, 0, s>>>(ex, nx, kNoExp);
-    crt_fill_kernel<<<64, 256, 0, s>>>(ey, ny, kNoExp);
+cudaError_t launch_crt_fill(int64_t n, int32_t *exps, cudaStream_t s) {
+    const int64_t want = (n + 255) / 256;
+    const int grid = (int)(want < 2 * num_sms() ? want : 2 * num_sms());
+    if (grid > 0) crt_fill_kernel<<<grid, 256, 0, s>>>(exps, (int32_t)n, kNoExp);
     return cudaGetLastError();
 }
 

@@ -212,10 +212,16 @@ struct CrtExec {
     int64_t exp_elems = 0;                  // elements the exponent pass reads (the others: per pass)
     int32_t sampled = 0;                    // sampled exponent bounds, checked by the residue pass
     double scale = 1.0;                     // kc (and d in add mode) times the pair coefficients' scale
-    DevBuf panels, units, tasks, items, cblks, comps, ctab, cells, gidx, ex, ey, res, out;
-    DevBuf cta_items;                       // products kernel: per-CTA item list offsets (ncta + 1)
+    DevBuf panels, units, tasks, items, cblks, comps, ctab, cells, gidx, exps, res, out;
+    DevBuf cta_items;                       // products kernel: per-CTA work lists
     int32_t ncta = 0;
-    DevBuf ext, eyt;                        // exact exponents of the sampled rows
+    // side tables in exps: row and column exponents, then their exact values
+    // where the residue pass forms them (sampled rows)
+    int32_t *ex() const { return exps.as<int32_t>(); }
+    int32_t *ey() const { return ex() + std::max<int32_t>(nx, 1); }
+    int32_t *ext() const { return ey() + std::max<int32_t>(ny, 1); }
+    int32_t *eyt() const { return ext() + std::max<int32_t>(nx, 1); }
+    int64_t nexps() const { return 2 * ((int64_t)std::max<int32_t>(nx, 1) + std::max<int32_t>(ny, 1)); }
     // row families split in one read (launch_crt_fused): families, their
     // panels and tile offsets, and the 8-row units
     DevBuf fams, famp, famt, funits;
@@ -1023,6 +1029,10 @@ SubDims fuse_single(int n, const int64_t *ext, const int64_t *str) {
     return r;
 }
 
+// Reading an accumulator back costs the products kernel about as much as this
+// many contracted elements (14 clocks per column against 1/64 per element).
+constexpr double kCrtDrainK = 900.0;
+
 int32_t round4(int64_t x) { return (int32_t)((x + 3) / 4 * 4); }
 
 // C dims of each side: connected to A (rows) or to B (columns), and the
@@ -1688,17 +1698,17 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
                 it.nx = xstep == 256 && x0 + 128 < q.xext ? 2 : 1;
                 it.t_begin = q.t_begin; it.t_end = q.t_end;
                 it.gx = q.gx; it.gy = q.gy;
-                iv.push_back({q.kw * q.nt * it.nx, it});
+                iv.push_back({(q.kw + kCrtDrainK) * q.nt * it.nx, it});
                 total_cost += iv.back().first;
             }
-    // a 256-row item costing more than one SM's share of the launch is cut
-    // into its two 128-row tiles (which load the N-side tile twice), so that
-    // no item alone outlasts the others
+    // Work is dealt per item and modulus (below); a 256-row item of which one
+    // modulus alone is more than half an SM's share of the launch is cut into its
+    // two 128-row tiles (which load the N-side tile twice)
     const int nsm = std::max(1, pl->ctx->nsm);
     {
         std::vector<std::pair<double, DCrtItem>> cut;
         for (auto &q : iv) {
-            if (q.second.nx == 2 && q.first > total_cost / nsm) {
+            if (q.second.nx == 2 && q.first > 0.5 * total_cost * L / nsm) {
                 DCrtItem a = q.second, b = q.second;
                 a.nx = b.nx = 1;
                 b.x0 += 128;
@@ -1728,19 +1738,53 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
         out_bytes += (int64_t)L * it.nx * 128 * it.nt;
         items.push_back(it);
     }
-    // Each persistent CTA of the products kernel works through its own list:
-    // the items, costliest first, dealt in waves of ncta in CTA order (items
-    // sharing an operand tile are adjacent in the order, so they run on
-    // neighbouring CTAs at the same time and share the tile through L2; with
-    // the cut above the waves balance.  Dealing every other wave in reverse
-    // order balanced the same on paper and ran the ladder's products 8 %
-    // slower).  cta_items holds the ncta + 1 list offsets (into itself), then
-    // the lists' item indexes.
-    const int32_t ncta = (int32_t)std::min<size_t>(items.size(), (size_t)nsm);
+    // Each persistent CTA of the products kernel works through its own list of
+    // (item, range of moduli).  Whole items, costliest first, are dealt in waves
+    // of ncta in CTA order (items sharing an operand tile are adjacent in the
+    // order, so they run on neighbouring CTAs at the same time and share the
+    // tile through L2; dealing every other wave in reverse order ran the ladder's
+    // products 8 % slower), as many full waves as keep every CTA within its share
+    // of the launch.  The other items are dealt one modulus at a time, each to
+    // the CTA with the least work so far: they would leave most SMs idle in a
+    // last wave (@FIG@).  cta_items holds the ncta + 1 list offsets (into
+    // itself), then the lists' pairs (item, first modulus | end modulus << 8).
+    const int32_t ncta = (int32_t)std::min<size_t>(items.size() * L, (size_t)nsm);
     std::vector<int32_t> cta_items;
     {
+        const size_t n = items.size();
         std::vector<std::vector<int32_t>> lists(std::max(ncta, 1));
-        for (size_t i = 0; i < items.size(); i++) lists[i % ncta].push_back((int32_t)i);
+        std::vector<double> load(std::max(ncta, 1), 0.0);
+        double total = 0;
+        for (const auto &q : iv) total += q.first * L;
+        size_t whole = 0;
+        double most = 0;                                 // CTA 0 takes the costliest item of each wave
+        while (whole + ncta <= n && (most += iv[whole].first * L) <= total / ncta) whole += ncta;
+        for (size_t i = 0; i < whole; i++) {
+            lists[i % ncta].push_back((int32_t)i);
+            lists[i % ncta].push_back(L << 8);
+            load[i % ncta] += iv[i].first * L;
+        }
+        typedef std::pair<double, int32_t> Load;
+        std::priority_queue<Load, std::vector<Load>, std::greater<Load>> least;
+        for (int32_t b = 0; b < ncta; b++) least.push({load[b], b});
+        // items of equal cost together, modulus by modulus, so that items sharing
+        // an operand tile stay on neighbouring CTAs
+        for (size_t i0 = whole, i1; i0 < n; i0 = i1) {
+            for (i1 = i0 + 1; i1 < n && iv[i1].first == iv[i0].first; i1++) {}
+            for (int32_t l = 0; l < L; l++)
+                for (size_t i = i0; i < i1; i++) {
+                    const Load x = least.top();
+                    least.pop();
+                    std::vector<int32_t> &v = lists[x.second];
+                    if (!v.empty() && v[v.size() - 2] == (int32_t)i && (v.back() >> 8) == l) {
+                        v.back() += 1 << 8;              // the next modulus of the CTA's last item
+                    } else {
+                        v.push_back((int32_t)i);
+                        v.push_back(l | (l + 1) << 8);
+                    }
+                    least.push({x.first + iv[i].first, x.second});
+                }
+        }
         cta_items.push_back(ncta + 1);
         for (int32_t b = 0; b < ncta; b++) cta_items.push_back(cta_items.back() + (int32_t)lists[b].size());
         for (int32_t b = 0; b < ncta; b++) cta_items.insert(cta_items.end(), lists[b].begin(), lists[b].end());
@@ -1846,10 +1890,7 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
     // cells of grouped images that no piece writes stay zero
     LTG_CUDA(cudaMemsetAsync(ex->res.p, 0, std::max<int64_t>(res_bytes, 1024), s));
     ex->out.alloc(std::max<int64_t>(out_bytes, 1024));
-    ex->ex.alloc(std::max<int64_t>(ex->nx, 1) * sizeof(int32_t));
-    ex->ey.alloc(std::max<int64_t>(ex->ny, 1) * sizeof(int32_t));
-    ex->ext.alloc(std::max<int64_t>(ex->nx, 1) * sizeof(int32_t));
-    ex->eyt.alloc(std::max<int64_t>(ex->ny, 1) * sizeof(int32_t));
+    ex->exps.alloc(ex->nexps() * sizeof(int32_t));
     upload_vec(ex->panels, panels, s);
     upload_vec(ex->tasks, dt, s);
     upload_vec(ex->items, items, s);
@@ -2521,19 +2562,18 @@ void run_crt(ltg_plan *plan, CrtExec *cx, double *carena, int add, const CrtDest
             LTG_CUDA(cudaMemsetAsync(carena + r.first, 0, (r.second - r.first) * sizeof(double), s));
     const double *pa = plan->a->arena.as<double>(), *pb = plan->b->arena.as<double>();
     TimedLaunch t_split(ctx, LTG_KERNEL_OZ_SPLIT);
-    LTG_CUDA(launch_crt_fill(cx->nx, cx->ny, cx->ex.as<int32_t>(), cx->ey.as<int32_t>(), s));
-    LTG_CUDA(launch_crt_fill(cx->nx, cx->ny, cx->ext.as<int32_t>(), cx->eyt.as<int32_t>(), s));
+    LTG_CUDA(launch_crt_fill(cx->nexps(), cx->ex(), s));
     LTG_CUDA(launch_crt_fused(plan->fused_split, cx->panels.as<DCrtPanel>(), cx->fams.as<DCrtFamily>(), cx->famp.as<int32_t>(),
                               cx->famt.as<int32_t>(), cx->funits.as<int4>(), cx->nfunits, pa, pb,
-                              cx->gidx.as<int32_t>(), cx->ex.as<int32_t>(), cx->ey.as<int32_t>(),
+                              cx->gidx.as<int32_t>(), cx->ex(), cx->ey(),
                               cx->res.as<uint8_t>(), cx->cp, s));
     LTG_CUDA(launch_crt_exponents(cx->panels.as<DCrtPanel>(), cx->units.as<int4>(), cx->nunits, cx->nx,
-                                  cx->ny, pa, pb, cx->gidx.as<int32_t>(), cx->ex.as<int32_t>(),
-                                  cx->ey.as<int32_t>(), cx->sampled, s));
+                                  cx->ny, pa, pb, cx->gidx.as<int32_t>(), cx->ex(),
+                                  cx->ey(), cx->sampled, s));
     for (int redo = 0; redo <= cx->sampled; redo++)
         LTG_CUDA(launch_crt_residues(cx->panels.as<DCrtPanel>(), cx->units.as<int4>(), cx->nunits, pa, pb,
-                                     cx->gidx.as<int32_t>(), cx->ex.as<int32_t>(), cx->ey.as<int32_t>(),
-                                     cx->ext.as<int32_t>(), cx->eyt.as<int32_t>(), cx->sampled, redo,
+                                     cx->gidx.as<int32_t>(), cx->ex(), cx->ey(),
+                                     cx->ext(), cx->eyt(), cx->sampled, redo,
                                      cx->res.as<uint8_t>(), cx->cp, s));
     t_split.done();
     TimedLaunch t_gemm(ctx, LTG_KERNEL_OZ_GEMM);
@@ -2546,11 +2586,11 @@ void run_crt(ltg_plan *plan, CrtExec *cx, double *carena, int add, const CrtDest
     LTG_CUDA(launch_crt_combine(cx->panels.as<DCrtPanel>(), cx->items.as<DCrtItem>(), cx->nitems,
                                 cx->cblks.as<DCBlock>(), cx->comps.as<DCrtComp>(), cx->ctab.as<int32_t>(),
                                 cx->cells.as<DCrtCell>(), cx->out.as<uint8_t>(), cx->gidx.as<int32_t>(),
-                                cx->ex.as<int32_t>(), cx->ey.as<int32_t>(), cx->ext.as<int32_t>(),
-                                cx->eyt.as<int32_t>(), carena, add,
+                                cx->ex(), cx->ey(), cx->ext(),
+                                cx->eyt(), carena, add,
                                 cx->scale, cx->cp, s, dd));
     t_comb.done();
-    ctx->launches += 4 + (cx->nfunits > 0 ? 1 : 0) + (cx->nunits > 0 ? 2 + cx->sampled : 0) +
+    ctx->launches += 1 + (cx->nfunits > 0 ? 1 : 0) + (cx->nunits > 0 ? 2 + cx->sampled : 0) +
                      (cx->nitems > 0 ? 2 : 0);
     fetch_device_wait(ctx);
 }

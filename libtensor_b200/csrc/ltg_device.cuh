@@ -353,8 +353,9 @@ cudaError_t launch_crt_exponents(const DCrtPanel *panels, const int4 *units, int
     int32_t *ey, int32_t sample, cudaStream_t s);
 bool crt_unit_sampled(const DCrtPanel &p, int unit_map);
 int64_t crt_sampled_elems(const DCrtPanel &p);        // elements of one row the sampled pass reads
-// Sets both exponent tables to "no element" (before the passes below).
-cudaError_t launch_crt_fill(int32_t nx, int32_t ny, int32_t *ex, int32_t *ey, cudaStream_t s);
+// Sets n exponents (the side tables, which lie one after the other) to "no
+// element" (before the passes below).
+cudaError_t launch_crt_fill(int64_t n, int32_t *exps, cudaStream_t s);
 
 // Exponents and residues of the row families in one HBM read, in kernel
 // shape 1-4 (units: crt_fuse_rows(shape) rows of one family, {family, first
@@ -370,8 +371,9 @@ cudaError_t launch_crt_residues(const DCrtPanel *panels, const int4 *units, int3
     const double *a, const double *b, const int32_t *gidx, const int32_t *ex, const int32_t *ey,
     int32_t *ext, int32_t *eyt, int32_t sample, int32_t redo, uint8_t *res, const CrtParams &cp,
     cudaStream_t s);
-// Products: ncta persistent CTAs, CTA b working through the items
-// cta_items[j], j in [cta_items[b], cta_items[b + 1]).
+// Products: ncta persistent CTAs, CTA b working through the pairs
+// (item, first modulus | end modulus << 8) at cta_items[j], j in
+// [cta_items[b], cta_items[b + 1]).
 cudaError_t launch_crt_gemm(const DCrtPanel *panels, const uint8_t *res, const DCrtTask *tasks,
     const DCrtItem *items, const int32_t *cta_items, int32_t ncta, uint8_t *out, const CrtParams &cp, int32_t *err,
     uint64_t wait_ns, int32_t stage_kb, cudaStream_t s);
