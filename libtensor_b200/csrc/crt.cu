@@ -20,8 +20,8 @@
 //      reduce it mod m_l to one byte per element; items of one 128-row tile
 //      alternate between two accumulator slots, so that the MMA warp fills
 //      one with the next modulus while the epilogue drains the other;
-//   4. recombination (crt_combine_kernel): Garner's mixed-radix algorithm
-//      with balanced digits gives the exact integer sum_p c_p A'_p B'_p in
+//   4. recombination (crt_combine_kernel): the Chinese remainder theorem, with
+//      its weights in exact limbs, gives the integer sum_p c_p A'_p B'_p in
 //      (-M/2, M/2), M = prod m_l (the host chooses P so that it fits), which
 //      is scaled by 2^(e_row + e_col - 2P) and the contraction coefficient in
 //      FP64 and written to C (assign or add).
@@ -66,37 +66,36 @@ __host__ __device__ constexpr int32_t crt_modulus(int i) {
            i == 6 ? 239 : i == 7 ? 233 : i == 8 ? 229 : i == 9 ? 227 : i == 10 ? 223 : i == 11 ? 217 :
            i == 12 ? 211 : i == 13 ? 199 : i == 14 ? 197 : 193;
 }
-// m_j^-1 mod m_i (extended Euclid)
-__host__ __device__ constexpr int32_t crt_inverse(int j, int i) {
-    int64_t m = crt_modulus(i), t = 0, nt = 1, r = m, nr = crt_modulus(j) % m;
-    while (nr != 0) {
-        const int64_t q = r / nr;
-        const int64_t t2 = t - q * nt; t = nt; nt = t2;
-        const int64_t r2 = r - q * nr; r = nr; nr = r2;
-    }
-    return (int32_t)(t < 0 ? t + m : t);
+// Chinese-remainder reconstruction: X = sum_i r_i W_i mod M with M = prod m_i and
+// W_i = (M / m_i) ((M / m_i)^-1 mod m_i) < M.  The weights are cut into limbs of
+// kLimbBits bits, W_i = sum_n limb_n(i) 2^(kLimbBits n), so that each limb's sum
+// over at most 16 residues below 256 is an integer below 2^53, exact in FP64.
+constexpr int kLimbBits = 41;
+__host__ __device__ constexpr unsigned __int128 crt_product(int L) {
+    unsigned __int128 m = 1;
+    for (int i = 0; i < L; i++) m *= (unsigned)crt_modulus(i);
+    return m;
 }
-
-// Balanced representative of x mod m, in (-m/2, m/2].
-__host__ __device__ constexpr int32_t crt_balanced(int64_t x, int32_t m) {
-    const int64_t y = ((x % m) + m) % m;
-    return (int32_t)(y > m / 2 ? y - m : y);
+__host__ __device__ constexpr unsigned __int128 crt_weight(int L, int i) {
+    const unsigned __int128 w = crt_product(L) / (unsigned)crt_modulus(i);
+    unsigned inv = 1;
+    while ((unsigned)(w % (unsigned)crt_modulus(i)) * inv % (unsigned)crt_modulus(i) != 1) inv++;
+    return w * inv;
 }
-__host__ __device__ constexpr bool crt_odd_moduli() {
-    for (int i = 1; i < 16; i++)
-        if (crt_modulus(i) % 2 == 0) return false;
-    return true;
+__host__ __device__ constexpr int crt_limbs(int L) {
+    int n = 0;
+    for (unsigned __int128 m = crt_product(L); m != 0; m >>= kLimbBits) n++;
+    return n;
 }
-static_assert(crt_odd_moduli(), "the single-reduction Garner digits need odd moduli after m_0");
-// Garner's digit i as one linear form: the recurrence t <- (t - v_j) m_j^-1
-// (mod m_i), j = 0..i-1, started at t = r_i, expands to
-//   v_i = r_i * prod_{j<i} m_j^-1 - sum_{j<i} v_j * prod_{k=j..i-1} m_k^-1  (mod m_i),
-// so the digit costs i multiply-adds and one reduction.  The products are
-// taken balanced (|.| <= 128).
-__host__ __device__ constexpr int32_t crt_garner_d(int j, int i) {
-    int64_t p = 1;
-    for (int k = j; k < i; k++) p = p * crt_inverse(k, i) % crt_modulus(i);
-    return crt_balanced(p, crt_modulus(i));
+__host__ __device__ constexpr double crt_limb(unsigned __int128 x, int n) {
+    return (double)(unsigned long long)((x >> (kLimbBits * n)) & (((unsigned __int128)1 << kLimbBits) - 1));
+}
+// 2^(kLimbBits n) / M
+__host__ __device__ constexpr double crt_limb_share(int L, int n) {
+    double v = 1.0;
+    for (int k = 0; k < kLimbBits * n; k++) v *= 2.0;
+    for (int i = 0; i < L; i++) v /= (double)crt_modulus(i);
+    return v;
 }
 
 // Compile-time loop: f(std::integral_constant<int, I>) for I in [B, E).
@@ -640,24 +639,21 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 // K-major shared-memory descriptor without swizzle (8-row x 16-byte core
-// matrices; k halves 128 bytes apart, 8-row groups 256 bytes apart).
-__device__ __forceinline__ uint64_t smem_desc_kmajor(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);
-    d |= (uint64_t)(128 >> 4) << 16;
-    d |= (uint64_t)(256 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
+// matrices; k halves 128 bytes apart, 8-row groups 256 bytes apart).  Low word:
+// start address and leading offset in 16-byte units; high word, the same for
+// every tile: stride offset and descriptor version.
+constexpr uint32_t kDescHi = (256u >> 4) | (1u << 14);
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr) { return ((addr >> 4) & 0x3FFF) | ((128u >> 4) << 16); }
 // kind::i8: S32 accumulator, signed INT8 A and B, K-major, M = 128, N = nt.
 __device__ __forceinline__ uint32_t instr_desc_i8(int nt) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(kXRows >> 4) << 24);
 }
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0;\n"
-                 "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p; }"
-                 :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+// x and y: low words of the operands' descriptors.
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint32_t x, uint32_t y, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{ .reg .pred p; .reg .b64 a, b; mov.b64 a, {%1, %5}; mov.b64 b, {%2, %5};\n"
+                 "setp.ne.b32 p, %4, 0;\n"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %3, p; }"
+                 :: "r"(tmem_d), "r"(x), "r"(y), "r"(idesc), "r"(accumulate), "n"(kDescHi) : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
@@ -770,7 +766,7 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
             for (int j = j0; j < j1 && ok; j += 2) {
                 const DCrtItem item = items[cta_items[j]];
                 const int l0 = cta_items[j + 1] & 255, l1 = cta_items[j + 1] >> 8;
-                const uint32_t idesc = instr_desc_i8(item.nt);
+                const uint32_t idesc = instr_desc_i8(item.nt), ystep = (uint32_t)(item.nt * kKB) >> 4;
                 for (int l = l0; l < l1 && ok; l++) {
                     // a two-tile fill takes both slots, a one-tile fill slot rr
                     const int s0 = item.nx == 2 ? 0 : rr;
@@ -790,16 +786,27 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
                             tc_fence_after();
                             const int nsub = min(KB, nkb - kb);
                             // stage layout: [first M tile's k blocks][second's][N tile's]
-                            const uint32_t sbase = smem0 + st * (KB * kSubBytes);
-                            const uint32_t ybytes = (uint32_t)item.nt * kKB;
-                            for (int j = 0; j < nsub; j++) {
-                                const uint32_t a0 = sbase + j * kXTile;
-                                const uint64_t db = smem_desc_kmajor(sbase + 2 * KB * kXTile + j * ybytes);
-                                umma_i8(d0, smem_desc_kmajor(a0), db, idesc, acc);
-                                if (item.nx == 2)
-                                    umma_i8(tmem + kMaxNt, smem_desc_kmajor(a0 + KB * kXTile), db, idesc, acc);
-                                acc = 1;
+                            const uint32_t dx = desc_lo(smem0 + st * (KB * kSubBytes));
+                            const uint32_t dy = dx + (uint32_t)((2 * KB * kXTile) >> 4);
+                            // whole stages without a branch: descriptors built and
+                            // tests made per MMA cost the issuing thread 280 clocks
+                            // per k block against 208 of products
+                            if (item.nx == 2 && nsub == KB) {
+#pragma unroll
+                                for (int j = 0; j < KB; j++) {
+                                    umma_i8(d0, dx + (uint32_t)((j * kXTile) >> 4), dy + (uint32_t)j * ystep, idesc, j == 0 ? acc : 1u);
+                                    umma_i8(tmem + kMaxNt, dx + (uint32_t)(((KB + j) * kXTile) >> 4), dy + (uint32_t)j * ystep, idesc,
+                                            j == 0 ? acc : 1u);
+                                }
+                            } else {
+                                for (int j = 0; j < nsub; j++) {
+                                    const uint32_t a0 = dx + (uint32_t)((j * kXTile) >> 4), b0 = dy + (uint32_t)j * ystep;
+                                    umma_i8(d0, a0, b0, idesc, j == 0 ? acc : 1u);
+                                    if (item.nx == 2)
+                                        umma_i8(tmem + kMaxNt, a0 + (uint32_t)((KB * kXTile) >> 4), b0, idesc, j == 0 ? acc : 1u);
+                                }
                             }
+                            acc = 1;
                             umma_commit(&empty_bar[st]);
                             if (++st == stages) { st = 0; ph ^= 1; }
                         }
@@ -891,14 +898,49 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(smem_u32(smem)), "l"(gmem) : "memory");
 }
 
+// The integer X in (-M/2, M/2) with the residues byte(i) mod m_i, rounded to
+// FP64.  The limb sums S_n are exact, q = rint(sum_i r_i W_i / M) is found from
+// the two highest (the host keeps |X| at least 1e-9 M / 2 inside the range, far
+// more than their error), each S_n - q M_n is exact again (q < 2^12), and the
+// limbs join from the top, where only the result is rounded.
+// Bound by FP64 issue: about 60 operations at 13 moduli.  Garner's mixed-radix
+// digits in FP32 took 346 instructions per element of the ring and were issue
+// bound (@COMB@).
+template<int L, class F>
+__device__ __forceinline__ double crt_reconstruct(F &&byte) {
+    constexpr int NL = crt_limbs(L);
+    double S[NL];
+    StaticFor<0, L>::run([&](auto ii) {
+        constexpr int i = decltype(ii)::value;
+        constexpr unsigned __int128 W = crt_weight(L, i);
+        // byte -> double by bits (2^52 + r)
+        const double r = __hiloint2double(0x43300000, (int)byte(ii)) - 4503599627370496.0;
+        StaticFor<0, NL>::run([&](auto nn) {
+            constexpr int n = decltype(nn)::value;
+            constexpr double w = crt_limb(W, n);
+            S[n] = i == 0 ? r * w : fma(r, w, S[n]);
+        });
+    });
+    constexpr double c1 = crt_limb_share(L, NL - 1), c0 = NL > 1 ? crt_limb_share(L, NL - 2) : 0.0;
+    const double q = fma(S[NL - 1], c1, NL > 1 ? S[NL > 1 ? NL - 2 : 0] * c0 : 0.0) + kMagicD - kMagicD;
+    double X = 0.0;
+    StaticFor<0, NL>::run([&](auto nn) {
+        constexpr int n = NL - 1 - decltype(nn)::value;
+        constexpr double m = crt_limb(crt_product(L), n), up = (double)(1ll << kLimbBits);
+        const double d = fma(-q, m, S[n]);
+        X = n == NL - 1 ? d : fma(X, up, d);
+    });
+    return X;
+}
+
 constexpr int kCombCols = 16;                       // tile columns staged per pass
 
 // Units (work item, 128-row half, 16-column chunk): the residues of the
 // unit staged in shared memory together with, per tile row and column, its
 // exponent and its part of the C offset (one C block: the offsets of its row
 // and column; grouped products: the block and coordinates, combined with the
-// C block's strides per element); then one thread per element runs Garner
-// and writes C.
+// C block's strides per element); then the threads reconstruct the elements and
+// write C.
 // SCATTER: each element goes, by atomic adds into a zeroed result, to its C
 // block's destinations instead -- blocks of another tensor with their own
 // index mappings and coefficients (the terms of a symmetrizer over the
@@ -973,11 +1015,8 @@ crt_combine_kernel(const DCrtPanel *__restrict__ panels, const DCrtItem *__restr
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
-        for (int e = threadIdx.x; e < kXRows * kCombCols; e += blockDim.x) {
-            int r, c;
-            if (cp.swap) { r = e & (kXRows - 1); c = e >> 7; }      // C rows along the tile columns
-            else { c = e & (kCombCols - 1); r = e >> 4; }
-            if (r >= xr || c0 + c >= yc) continue;
+        // one element: row r and column c0 + c of the tile; byte(i) its residues
+        auto element = [&](int r, int c, auto &&byte) {
             int64_t off = 0;
             int cell = -1;
             const int32_t *cm = nullptr, *cn = nullptr;
@@ -986,7 +1025,7 @@ crt_combine_kernel(const DCrtPanel *__restrict__ panels, const DCrtItem *__restr
                 cm = cp.swap ? cy : cx;
                 cn = cp.swap ? cx : cy;
                 cell = ctab[cc->cell_off + cm[0] * cc->ncb + cn[0]];
-                if (cell < 0) continue;
+                if (cell < 0) return;
                 if constexpr (!SCATTER) {
                     const DCrtCell &cl = cells[cell];
                     off = cl.c_off;
@@ -996,37 +1035,7 @@ crt_combine_kernel(const DCrtPanel *__restrict__ panels, const DCrtItem *__restr
             } else if constexpr (!SCATTER) {
                 off = cb1->c_off + soff[r] + soff[kXRows + c];
             }
-            // Garner: balanced mixed-radix digits v_i of the residues.  Every
-            // quantity is an integer below 2^19 in magnitude (|r_i D| <=
-            // 255 * 128, |v_j D| <= 128 * 128, at most 15 terms), so FP32
-            // holds it exactly; the quotient rint(t / m_i) from one FMA is
-            // exact for odd m_i (t / m_i stays 1/(2 m_i) away from a half
-            // integer, far above the product's rounding), which leaves t
-            // in [-(m_i - 1)/2, (m_i - 1)/2].
-            float v[L];
-            StaticFor<0, L>::run([&](auto ii) {
-                constexpr int i = decltype(ii)::value;
-                const float ri = __int_as_float(0x4B000000 | (int)sres[i][r][c]) - 8388608.0f;
-                if constexpr (i == 0) {
-                    v[0] = ri >= 128.0f ? ri - 256.0f : ri;             // m_0 = 256: the byte itself
-                } else {
-                    constexpr float mi = (float)crt_modulus(i), minv = 1.0f / (float)crt_modulus(i);
-                    float t = ri * (float)crt_garner_d(0, i);
-                    StaticFor<0, i>::run([&](auto jj) {
-                        constexpr int j = decltype(jj)::value;
-                        t = fmaf(-v[j], (float)crt_garner_d(j, i), t);
-                    });
-                    v[i] = fmaf(-(fmaf(t, minv, kMagicF) - kMagicF), mi, t);
-                }
-            });
-            // digits to double by bits (|v| < 2^22): float 1.5*2^23 + v -> int -> double
-            auto digit = [](float f) {
-                const int iv = __float_as_int(f + kMagicF) - 0x4B400000;
-                return __hiloint2double(0x43380000, iv ^ (int)0x80000000) - 6755401588539392.0;
-            };
-            double X = digit(v[L - 1]);
-#pragma unroll
-            for (int i = L - 2; i >= 0; i--) X = fma(X, (double)crt_modulus(i), digit(v[i]));
+            const double X = crt_reconstruct<L>(byte);
             // 2^(e_row + e_col - 2P) from its bits (a row without exponent has X = 0)
             const int e2 = sexp[r] + sexp[kXRows + c] - 2 * cp.P;
             const double p2 = e2 < -1022 ? 0.0 : __hiloint2double((min(e2, 1023) + 1023) << 20, 0);
@@ -1050,6 +1059,29 @@ crt_combine_kernel(const DCrtPanel *__restrict__ panels, const DCrtItem *__restr
                 double *dst = C + off;
                 if (add) *dst += val;
                 else *dst = val;
+            }
+        };
+        if (cp.swap) {
+            // C rows along the tile columns, so C is contiguous along the tile
+            // rows: a row and four columns per thread, whose residues of a
+            // modulus are one word (single bytes 16 apart would hit each bank
+            // four times)
+            for (int e = threadIdx.x; e < kXRows * (kCombCols / 4); e += blockDim.x) {
+                const int r = e & (kXRows - 1), c = (e >> 7) * 4;
+                if (r >= xr || c0 + c >= yc) continue;
+                uint32_t w[L];
+#pragma unroll
+                for (int i = 0; i < L; i++) w[i] = *reinterpret_cast<const uint32_t *>(&sres[i][r][c]);
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (c0 + c + j < yc)
+                        element(r, c + j, [&](auto ii) { return (w[decltype(ii)::value] >> (8 * j)) & 255u; });
+            }
+        } else {
+            for (int e = threadIdx.x; e < kXRows * kCombCols; e += blockDim.x) {
+                const int c = e & (kCombCols - 1), r = e >> 4;
+                if (r >= xr || c0 + c >= yc) continue;
+                element(r, c, [&](auto ii) { return (uint32_t)sres[decltype(ii)::value][r][c]; });
             }
         }
     }

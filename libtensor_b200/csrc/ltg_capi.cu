@@ -1568,7 +1568,8 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
     // |c * x * 2^(P - e)| < 2^50 keeps every residue computation exact (the
     // FP64 round-to-integer trick needs magnitudes below 2^51)
     const int pcap = 50 - (int)std::ceil(std::log2((double)max_coef));
-    const int P = std::min(pcap, (int)std::floor((log2M - 1.0 - std::log2((double)max_sum)) / 2.0));
+    // (1e-9 inside the range: the recombination finds X / M in FP64)
+    const int P = std::min(pcap, (int)std::floor((log2M - 1.0 - 1e-9 - std::log2((double)max_sum)) / 2.0));
     if (P < 24) throw error(kErrUnsupported, "too few moduli for this contraction");
 
     std::unique_ptr<CrtExec> ex(new CrtExec());
@@ -1743,11 +1744,16 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
     // of ncta in CTA order (items sharing an operand tile are adjacent in the
     // order, so they run on neighbouring CTAs at the same time and share the
     // tile through L2; dealing every other wave in reverse order ran the ladder's
-    // products 8 % slower), as many full waves as keep every CTA within its share
-    // of the launch.  The other items are dealt one modulus at a time, each to
-    // the CTA with the least work so far: they would leave most SMs idle in a
-    // last wave (@FIG@).  cta_items holds the ncta + 1 list offsets (into
-    // itself), then the lists' pairs (item, first modulus | end modulus << 8).
+    // products 8 % slower).  Where that leaves the fullest CTA more than 10 % above
+    // its share of the launch, only as many full waves as keep within the share
+    // are dealt so, and the other items one modulus at a time, each to the CTA
+    // with the least work so far: a contraction with fewer items than SMs would
+    // leave most of them idle (ladder o=20 v=90, 43 items: 158 us whole, 46 by
+    // modulus; ring D2h o=46 v=296, 202 uneven items: 195 and 144).  Below 10 % the
+    // sharing is worth more: the ladder o=40 v=240 (566 items, 8 % over) ran
+    // 1.79 ms whole on every GPU, and 1.78 to 2.06 by modulus depending on it.
+    // cta_items holds the ncta + 1 list offsets (into itself), then the lists'
+    // pairs (item, first modulus | end modulus << 8).
     const int32_t ncta = (int32_t)std::min<size_t>(items.size() * L, (size_t)nsm);
     std::vector<int32_t> cta_items;
     {
@@ -1756,8 +1762,11 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
         std::vector<double> load(std::max(ncta, 1), 0.0);
         double total = 0;
         for (const auto &q : iv) total += q.first * L;
+        // CTA 0 takes the costliest item of each wave
         size_t whole = 0;
-        double most = 0;                                 // CTA 0 takes the costliest item of each wave
+        double most = 0, all = 0;
+        for (size_t i = 0; i < n; i += ncta) all += iv[i].first * L;
+        if (all <= 1.1 * total / ncta) whole = n;
         while (whole + ncta <= n && (most += iv[whole].first * L) <= total / ncta) whole += ncta;
         for (size_t i = 0; i < whole; i++) {
             lists[i % ncta].push_back((int32_t)i);

@@ -182,7 +182,7 @@ struct DCrtCell {
     int32_t ms[kCrtSideDims], ns[kCrtSideDims];
 };
 
-// Moduli of a modular contraction and its scaling (the constants of Garner's
+// Moduli of a modular contraction and its scaling (the constants of the
 // reconstruction are compile-time functions of the same moduli in crt.cu).
 struct CrtParams {
     int32_t L;                    // number of moduli
@@ -343,7 +343,7 @@ double oz_product_cost(int64_t x, int64_t y, int S);
 void oz_kind_params(int kind, int *beta0, int *beta, int *esz, int *kbe, int64_t *maxprod);
 
 // Modular split precision: exponent pass, residue pass, modular products,
-// Garner recombination into FP64 C.
+// recombination into FP64 C.
 // Split passes work on units (panel, first row, rows, unused): at most 256
 // rows of one panel.
 // sample != 0: long rows of row-mapped units (crt_unit_sampled) contribute
@@ -390,7 +390,7 @@ struct CrtDests {
     const DCrtCell *gdcells;
     const double *gdcoef;
 };
-// Garner recombination into C; each row's exponent is max(ex, ext) (the
+// Recombination into C; each row's exponent is max(ex, ext) (the
 // bound, or the exact exponent of a row the residue pass redid).  With dd,
 // each element is added atomically to its destinations instead (c zeroed
 // before; add ignored).

@@ -47,3 +47,31 @@ def test_redone_rows_take_their_short_panels_along(vir):
     for x in (op, P, C, A, B):
         x.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("moduli", range(8, 17))
+@pytest.mark.parametrize("m,n", [(300, 40), (37, 259), (1, 130)], ids=["rows long", "columns long", "one row"])
+def test_recombination_is_exact_on_integers(moduli, m, n):
+    """Integers below 2^11 are exact in the P >= 24 bits of every modulus count
+    and 100 of their products stay below 2^53, so the recombined result must
+    equal the integer result, either side along the tile rows; the last terms
+    cancel in one column, whose exact zeros must come out as zeros."""
+    ctx = Context(0)
+    rng = np.random.default_rng(moduli)
+    a = rng.integers(-2047, 2048, (m, 100)).astype(float)
+    b = rng.integers(-2047, 2048, (n, 100)).astype(float)
+    b[n // 2] = 0.0
+    b[n // 2, :2], a[:, 1] = (1.0, -1.0), a[:, 0]
+    A = block_tensor(ctx, S.BTSpec(dims=[m, 100], splits=[[], [60]]))
+    B = block_tensor(ctx, S.BTSpec(dims=[n, 100], splits=[[], [60]]))
+    for t, x in ((A, a), (B, b)):
+        t.set_block((0, 0), x[:, :60])
+        t.set_block((0, 1), x[:, 60:])
+    op = btod_contract2(contraction2(1, 1, 1).contract(1, 1), A, B)
+    C = op.make_result()
+    op.perform(C, mode=MODE_OZAKI_CRT, nslices=moduli)
+    ctx.synchronize()
+    assert np.array_equal(C.get_block((0, 0), (m, n)), a @ b.T)
+    for x in (op, C, A, B):
+        x.close()
+    ctx.close()
