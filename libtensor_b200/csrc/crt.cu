@@ -28,9 +28,9 @@
 // The error is that of rounding each operand to P bits relative to its row's
 // largest element (P about 43 for 13 moduli and K up to a few thousand).
 //
-// Warp roles of the products kernel (320 threads): warps 0-7 epilogue (two
-// per TMEM lane quarter, one tile row per thread, alternate 16-column
-// chunks), warp 8 bulk-copy producer, warp 9 MMA issuer.  Operand tiles are whole tile images moved by 1-D
+// Warp roles of the products kernel (576 threads): warps 0-15 epilogue (four
+// per TMEM lane quarter, one tile row per thread, every fourth 16-column
+// chunk), warp 16 bulk-copy producer, warp 17 MMA issuer.  Operand tiles are whole tile images moved by 1-D
 // cp.async.bulk (no tensor maps, no multicast); every mbarrier wait is
 // bounded in time and reports through *err.
 #include <type_traits>
@@ -49,7 +49,11 @@ constexpr int kSubBytes = 2 * kXTile + kMaxNt * kKB;    // one k block: two M ti
 // (a stage holds KB k blocks as [M tile 0][M tile 1][N tile] regions; KB is
 // the products kernel's template parameter, crt_stage_kb() at launch)
 constexpr int kMaxStages = 8;
-constexpr int kEpiWarps = 8;                        // two per TMEM lane quarter
+// Four epilogue warps per TMEM lane quarter: with two, reading back a modulus
+// (2 x 128 x 208 sums, 5,700 clocks) held the ring's short products for 41 % of
+// their time; four run the ring in 143 us (148), the ladder o=40 v=240 in 1.74 ms
+// (1.76).
+constexpr int kEpiWarps = 16;
 constexpr int kGemmThreads = 32 * (kEpiWarps + 2);  // + bulk-copy producer + MMA issuer
 constexpr uint64_t kWaitNs = 2000000000ull;         // 2 s: the drain waits after an abort
 constexpr double kMagicD = 6755399441055744.0;      // 1.5 * 2^52: round-to-integer constant
@@ -827,9 +831,9 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
             }
         }
     } else {
-        // ------------------------------------------------ epilogue (warps 0-7)
+        // ------------------------------------------------ epilogue (warps 0-15)
         // warp w reads TMEM lanes 32 (w % 4) .. + 31 (the lane quarter a warp
-        // may access) and every other 16-column chunk, starting at 16 (w / 4)
+        // may access) and every fourth 16-column chunk, starting at 16 (w / 4)
         const int quarter = warp & 3, chunk0 = (warp >> 2) * 16;
         const int row = quarter * 32 + lane;                      // TMEM lane == tile row
         uint32_t uses[2] = {0, 0};                                // same slot sequence as the MMA warp
@@ -849,7 +853,7 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
                 for (int xh = 0; xh < item.nx; xh++) {
                     const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((s0 + xh) * kMaxNt);
                     uint8_t *orow = out + item.res_off + ((int64_t)(l * item.nx + xh) * kXRows + row) * item.nt;
-                    for (int c0 = chunk0; c0 < item.nt; c0 += 32) {
+                    for (int c0 = chunk0; c0 < item.nt; c0 += 4 * kEpiWarps) {
                         uint32_t v[16];
                         tmem_ld16(taddr + (uint32_t)c0, v);
                         tmem_wait_ld();
@@ -905,7 +909,8 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 // limbs join from the top, where only the result is rounded.
 // Bound by FP64 issue: about 60 operations at 13 moduli.  Garner's mixed-radix
 // digits in FP32 took 346 instructions per element of the ring and were issue
-// bound (@COMB@).
+// bound (170 us; 134 us this way; ladder o=40 v=240:
+// 226 to 161 us).
 template<int L, class F>
 __device__ __forceinline__ double crt_reconstruct(F &&byte) {
     constexpr int NL = crt_limbs(L);
