@@ -316,6 +316,80 @@ transfer_kernel(const DJob *__restrict__ jobs, const DTerm *__restrict__ terms,
     }
 }
 
+// Direct mode (jobs with a transposing term and small planes): a warp takes a
+// plane in steps of (32 >> vec) rows x (1 << vec) columns, every term read
+// straight from global memory.  With 4 x 8 a step covers 64-byte runs along the
+// destination's columns and 32-byte runs along a transposing source's rows;
+// what a misaligned run leaves of a sector the next steps find in L1.  Bound by
+// L1's lines per request, 1.6 to 2.8 TB/s, where staged tiles reach 3.3 to 6.3;
+// but a tile of a few hundred elements costs the staging CTA two barriers and a
+// copy latency.  Antisymmetriser o=10,6 v=21,24 (4 terms, 50 MB): 144 us staged,
+// 30 direct; copy P(1,0,3,2) v=13,11,6: 175 and 22 us.
+template<int NT>
+__global__ void __launch_bounds__(kThreads)
+transfer_direct_kernel(const DJob *__restrict__ jobs, const DTerm *__restrict__ terms,
+                       const DUnit *__restrict__ units, int32_t nunits,
+                       const double *const *__restrict__ srcs, double *__restrict__ dst,
+                       int32_t accumulate, double beta) {
+    constexpr int RU = NT <= 2 ? 8 : 4;                     // column steps in flight
+    __shared__ UnitDesc<NT> sd;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+        const DUnit un = units[u];
+        stage_unit<NT>(jobs, terms, un.job, sd);
+        const int nt = sd.j.nterms, dq = sd.j.dq;
+        const int lc = sd.j.vec, la = lane >> lc, lb = lane & ((1 << lc) - 1);
+        const int arows = 32 >> lc, bcols = 1 << lc;
+        const double *sp[NT];
+        double cf[NT];
+        int32_t sb[NT], sq[NT];
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+            sp[t] = t < nt ? srcs[sd.t[t].src] : nullptr;
+            cf[t] = t < nt ? sd.t[t].coeff : 0.0;
+            sb[t] = t < nt ? sd.t[t].sb : 0;
+            sq[t] = t < nt ? sd.t[t].sq : 0;
+        }
+        for (int64_t v = un.row_begin + warp; v < un.row_end; v += kWarps) {
+            int64_t db, sbase[NT];
+            int b0, na, nb;
+            tile_bases<NT>(sd, (uint32_t)v, db, sbase, b0, na, nb);
+            const double *p[NT];
+#pragma unroll
+            for (int t = 0; t < NT; t++) p[t] = sp[t] + sbase[t] + (int64_t)(b0 + lb) * sb[t] + (int64_t)la * sq[t];
+            double *d = dst + db + b0 + lb + (int64_t)la * dq;
+            for (int a = la; a - la < na; a += arows) {
+                for (int c = 0; c < nb; c += bcols * RU) {
+                    double val[RU];
+                    bool ok[RU];
+#pragma unroll
+                    for (int k = 0; k < RU; k++) {
+                        val[k] = 0.0;
+                        ok[k] = a < na && c + k * bcols + lb < nb;
+                    }
+#pragma unroll
+                    for (int t = 0; t < NT; t++) {
+                        if (t >= nt) break;
+#pragma unroll
+                        for (int k = 0; k < RU; k++)
+                            if (ok[k]) val[k] += cf[t] * p[t][(c + k * bcols) * sb[t]];
+                    }
+#pragma unroll
+                    for (int k = 0; k < RU; k++) {
+                        if (!ok[k]) continue;
+                        double *o = d + c + k * bcols;
+                        if (accumulate) *o = *o + beta * val[k];
+                        else *o = val[k];
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < NT; t++) p[t] += (int64_t)arows * sq[t];
+                d += (int64_t)arows * dq;
+            }
+        }
+    }
+}
+
 // Tiled mode (jobs with a transposing term): one CTA per tile at a time; every
 // term's tile is staged through shared memory, then combined in term order
 // and written along the destination's columns.
@@ -648,7 +722,7 @@ int grid_for(int64_t units) {
 
 template<int NT>
 cudaError_t launch_transfer_nt(const DJob *jobs, const DTerm *terms, const DUnit *units, int32_t nrow,
-                               int32_t ntiled, size_t smem, const double *const *srcs, double *dst,
+                               int32_t ntiled, int32_t ndirect, size_t smem, const double *const *srcs, double *dst,
                                int32_t accumulate, double beta, cudaStream_t s) {
     if (nrow > 0)
         transfer_kernel<NT><<<grid_for(nrow), kThreads, 0, s>>>(jobs, terms, units, nrow, srcs, dst,
@@ -665,22 +739,25 @@ cudaError_t launch_transfer_nt(const DJob *jobs, const DTerm *terms, const DUnit
         transfer_tiled_kernel<NT><<<grid_for(ntiled), kTiledThreads, bytes, s>>>(
             jobs, terms, units + nrow, ntiled, srcs, dst, accumulate, beta, stride);
     }
+    if (ndirect > 0)
+        transfer_direct_kernel<NT><<<grid_for(ndirect), kThreads, 0, s>>>(jobs, terms, units + nrow + ntiled, ndirect,
+                                                                          srcs, dst, accumulate, beta);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_transfer(const DJob *jobs, const DTerm *terms, const DUnit *units,
-                            int32_t nrow, int32_t ntiled, int32_t max_terms, int32_t tile_bytes,
+                            int32_t nrow, int32_t ntiled, int32_t ndirect, int32_t max_terms, int32_t tile_bytes,
                             const double *const *srcs, double *dst, int32_t accumulate, double beta,
                             cudaStream_t s) {
-    if (nrow + ntiled <= 0) return cudaSuccess;
+    if (nrow + ntiled + ndirect <= 0) return cudaSuccess;
     const size_t smem = (size_t)tile_bytes;
-    if (max_terms <= 1) return launch_transfer_nt<1>(jobs, terms, units, nrow, ntiled, smem, srcs, dst, accumulate, beta, s);
-    if (max_terms <= 2) return launch_transfer_nt<2>(jobs, terms, units, nrow, ntiled, smem, srcs, dst, accumulate, beta, s);
-    if (max_terms <= 4) return launch_transfer_nt<4>(jobs, terms, units, nrow, ntiled, smem, srcs, dst, accumulate, beta, s);
+    if (max_terms <= 1) return launch_transfer_nt<1>(jobs, terms, units, nrow, ntiled, ndirect, smem, srcs, dst, accumulate, beta, s);
+    if (max_terms <= 2) return launch_transfer_nt<2>(jobs, terms, units, nrow, ntiled, ndirect, smem, srcs, dst, accumulate, beta, s);
+    if (max_terms <= 4) return launch_transfer_nt<4>(jobs, terms, units, nrow, ntiled, ndirect, smem, srcs, dst, accumulate, beta, s);
     if (max_terms <= kMaxTerms)
-        return launch_transfer_nt<kMaxTerms>(jobs, terms, units, nrow, ntiled, smem, srcs, dst, accumulate, beta, s);
+        return launch_transfer_nt<kMaxTerms>(jobs, terms, units, nrow, ntiled, ndirect, smem, srcs, dst, accumulate, beta, s);
     return cudaErrorInvalidValue;
 }
 

@@ -1966,18 +1966,35 @@ void validate_transfer(const TransferPlan &plan, const std::vector<int64_t> &src
 struct DeviceTransfer {
     std::vector<DJob> jobs;
     std::vector<DTerm> terms;
-    std::vector<DUnit> units;          // row-mode units, then tiled-mode units
-    int32_t nrow = 0, ntiled = 0;
+    std::vector<DUnit> units;          // row-mode units, then tiled-mode, then direct-mode units
+    int32_t nrow = 0, ntiled = 0, ndirect = 0;
     int32_t max_terms = 0, tile_bytes = 0;
 };
 constexpr int64_t kTransferUnitElems = 32768;
 constexpr int32_t kItemElems = 4096;       // row mode: elements per warp item (about)
 constexpr int32_t kTileSide = 64;          // largest tile side (elements)
+// Direct mode: planes below this many elements.  Copy P(1,0,3,2), planes of 32 x
+// 30 to 32 x 32: 155 us staged, 140 direct; of 37 x 41: 267 and 394; the four-term
+// antisymmetriser, 30 x 33: 110 and 74 us, 50 x 50: 221 and 425.
+constexpr int64_t kDirectPlane = 1024;
 constexpr int64_t kTileSmemDoubles = 12288; // tiled mode: shared memory for all terms' tiles (96 KiB)
 
-DeviceTransfer device_transfer(const TransferPlan &plan, int64_t unit_elems = kTransferUnitElems) {
+// unit_elems: elements per unit of a large transfer; a small one has units of
+// 1024 elements or more, about 16 per SM, so that it fills the GPU.  direct:
+// transposing jobs with planes below kDirectPlane elements take the direct mode.
+DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, int64_t unit_elems = kTransferUnitElems) {
     DeviceTransfer o;
-    std::vector<DUnit> tiled_units;
+    std::vector<DUnit> tiled_units, direct_units;
+    int64_t total = 0;
+    for (const TJob &j : plan.jobs) {
+        int64_t n = 1;
+        for (int d = 0; d < j.ndim; d++) n *= j.ext[d];
+        total += n;
+    }
+    nsm = std::max(1, nsm);
+    unit_elems = std::min(unit_elems, std::max<int64_t>(1024, total / (16 * nsm)));
+    // row mode: likewise down to 256 elements per warp item, 64 items per SM
+    const int32_t item_elems = (int32_t)std::min<int64_t>(kItemElems, std::max<int64_t>(256, total / (64 * nsm)));
     for (const TJob &j : plan.jobs) {
         const int n = j.ndim, L = n - 1;
         const TTerm *T = plan.terms.data() + j.term0;
@@ -2012,10 +2029,10 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int64_t unit_elems = kT
             dj.odst[dj.nout] = (int32_t)dstr[d];
             dj.nout++;
         }
-        dj.tiled = transposing ? 1 : 0;
-        dj.seg = dj.B > kItemElems ? kItemElems : dj.B;
+        dj.tiled = !transposing ? 0 : direct && (int64_t)dj.A * dj.B < kDirectPlane ? 2 : 1;
+        dj.seg = dj.B > item_elems ? item_elems / 2 * 2 : dj.B;
         dj.nseg = (dj.B + dj.seg - 1) / dj.seg;
-        dj.ra = std::max<int32_t>(1, std::min<int32_t>(dj.A, kItemElems / dj.seg));
+        dj.ra = std::max<int32_t>(1, std::min<int32_t>(dj.A, item_elems / dj.seg));
         dj.nra = (dj.A + dj.ra - 1) / dj.ra;
         bool vec = !transposing && dj.seg % 2 == 0 && dj.B % 2 == 0 && dj.dst_off % 2 == 0 && dj.dq % 2 == 0;
         for (int k = 0; k < dj.nout; k++) vec = vec && dj.odst[k] % 2 == 0;
@@ -2025,6 +2042,13 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int64_t unit_elems = kT
         while (side > 8 && (int64_t)std::max(1, j.nterms) * side * (side + 1) > kTileSmemDoubles) side--;
         dj.nta = (dj.A + side - 1) / side;
         dj.ntb = (dj.B + side - 1) / side;
+        // (direct mode: down to steps of four rows where whole planes would not
+        // occupy 16 warps per SM)
+        if (dj.tiled == 2) {
+            const int64_t want = std::min<int64_t>((dj.A + 3) / 4, (int64_t)dj.A * dj.B * 16 * nsm / std::max<int64_t>(1, total));
+            const int32_t rows = (int32_t)((dj.A + std::max<int64_t>(dj.nta, want) - 1) / std::max<int64_t>(dj.nta, want));
+            dj.nta = (dj.A + rows - 1) / rows;               // no empty tile
+        }
         const int32_t ta_ext = (dj.A + dj.nta - 1) / dj.nta, tb_ext = (dj.B + dj.ntb - 1) / dj.ntb;
         int32_t toff = 0;
         for (int t = 0; t < j.nterms; t++) {
@@ -2054,9 +2078,19 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int64_t unit_elems = kT
             }
             o.terms.push_back(dt);
         }
-        dj.vec = vec ? 1 : 0;
+        int32_t lanes = 3;
+        if (dj.tiled == 2) {
+            // the lane shape with the fewest steps per plane, 4 x 8 unless another
+            // saves a fifth of them
+            int64_t best = INT64_MAX;
+            for (int32_t l : {3, 2, 4, 1, 5, 0}) {
+                const int64_t steps = (int64_t)((ta_ext + (32 >> l) - 1) / (32 >> l)) * ((tb_ext + (1 << l) - 1) >> l);
+                if (best == INT64_MAX || steps * 10 < best * 8) { best = steps; lanes = l; }
+            }
+        }
+        dj.vec = dj.tiled == 2 ? lanes : vec ? 1 : 0;
         o.max_terms = std::max(o.max_terms, j.nterms);
-        if (transposing) o.tile_bytes = std::max<int32_t>(o.tile_bytes, (toff + 1) * (int32_t)sizeof(double));
+        if (dj.tiled == 1) o.tile_bytes = std::max<int32_t>(o.tile_bytes, (toff + 1) * (int32_t)sizeof(double));
         const int32_t ji = (int32_t)o.jobs.size();
         o.jobs.push_back(dj);
         int64_t planes = 1;
@@ -2067,7 +2101,8 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int64_t unit_elems = kT
         if (dj.tiled) {
             items = planes * dj.nta * dj.ntb;
             const int64_t tile = (int64_t)((dj.A + dj.nta - 1) / dj.nta) * ((dj.B + dj.ntb - 1) / dj.ntb);
-            per_unit = std::max<int64_t>(1, unit_elems / tile);
+            // (direct mode: whole rounds of the CTA's eight warps)
+            per_unit = dj.tiled == 2 ? std::max<int64_t>(8, unit_elems / tile / 8 * 8) : std::max<int64_t>(1, unit_elems / tile);
         } else {
             items = planes * dj.nra * dj.nseg;
             const int64_t item = (int64_t)dj.ra * dj.seg;
@@ -2078,18 +2113,20 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int64_t unit_elems = kT
             u.job = ji;
             u.row_begin = r;
             u.row_end = std::min(items, r + per_unit);
-            (dj.tiled ? tiled_units : o.units).push_back(u);
+            (dj.tiled == 2 ? direct_units : dj.tiled == 1 ? tiled_units : o.units).push_back(u);
         }
     }
     o.nrow = (int32_t)o.units.size();
     o.ntiled = (int32_t)tiled_units.size();
+    o.ndirect = (int32_t)direct_units.size();
     o.units.insert(o.units.end(), tiled_units.begin(), tiled_units.end());
+    o.units.insert(o.units.end(), direct_units.begin(), direct_units.end());
     return o;
 }
 
 struct TransferExec {
     DevBuf jobs, terms, units, srcs;
-    int32_t nrow = 0, ntiled = 0, max_terms = 0, tile_bytes = 0;
+    int32_t nrow = 0, ntiled = 0, ndirect = 0, max_terms = 0, tile_bytes = 0;
     std::vector<char> dst_nonzero;
 };
 typedef std::tuple<std::vector<const ltg_bt *>, std::vector<int8_t>, std::vector<double>,
@@ -2128,7 +2165,7 @@ void run_transfer(ltg_ctx *ctx, const std::vector<ltg_bt *> &srcs, const std::ve
         for (ltg_bt *b : srcs) ssz.push_back(b->h.total_elems);
         validate_transfer(plan, ssz, dst->h.total_elems);
         std::unique_ptr<TransferExec> nx(new TransferExec());
-        DeviceTransfer dt = device_transfer(plan);
+        DeviceTransfer dt = device_transfer(plan, ctx->nsm, true);
         upload_vec(nx->jobs, dt.jobs, s);
         upload_vec(nx->terms, dt.terms, s);
         upload_vec(nx->units, dt.units, s);
@@ -2137,6 +2174,7 @@ void run_transfer(ltg_ctx *ctx, const std::vector<ltg_bt *> &srcs, const std::ve
         upload_vec(nx->srcs, sp, s);
         nx->nrow = dt.nrow;
         nx->ntiled = dt.ntiled;
+        nx->ndirect = dt.ndirect;
         nx->max_terms = dt.max_terms;
         nx->tile_bytes = dt.tile_bytes;
         nx->dst_nonzero = plan.dst_nonzero;
@@ -2146,7 +2184,7 @@ void run_transfer(ltg_ctx *ctx, const std::vector<ltg_bt *> &srcs, const std::ve
     }
     TimedLaunch tl(ctx, LTG_KERNEL_TRANSFER);
     LTG_CUDA(launch_transfer(ex->jobs.as<DJob>(), ex->terms.as<DTerm>(), ex->units.as<DUnit>(),
-                             ex->nrow, ex->ntiled, ex->max_terms, ex->tile_bytes, ex->srcs.as<const double *>(), dst->arena.as<double>(),
+                             ex->nrow, ex->ntiled, ex->ndirect, ex->max_terms, ex->tile_bytes, ex->srcs.as<const double *>(), dst->arena.as<double>(),
                              add ? 1 : 0, d, s));
     tl.done();
     ctx->launches++;
@@ -2187,7 +2225,7 @@ DotExec *prepare_dot(ltg_bt *a, const Perm &pa, ltg_bt *b, const Perm &pb) {
     std::unique_ptr<DotExec> ex(new DotExec());
     cudaStream_t s = a->ctx->stream;
     // larger units for the dot product: each unit ends in a CTA reduction
-    DeviceTransfer dt = device_transfer(plan, 4 * kTransferUnitElems);
+    DeviceTransfer dt = device_transfer(plan, a->ctx->nsm, false, 4 * kTransferUnitElems);
     upload_vec(ex->jobs, dt.jobs, s);
     upload_vec(ex->terms, dt.terms, s);
     upload_vec(ex->units, dt.units, s);

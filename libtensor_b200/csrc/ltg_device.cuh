@@ -222,11 +222,12 @@ struct DJob {
     int32_t dq;                   // destination stride of dim q
     int32_t nout;                 // outer dims, outermost first
     int32_t oext[kDevMaxOrder - 2], odst[kDevMaxOrder - 2];
-    int32_t vec;                  // 16-byte accesses valid for every term
+    int32_t vec;                  // row mode: 16-byte accesses valid for every term; direct mode: a
+                                  // warp steps 32 >> vec rows x 1 << vec columns
     int32_t seg, nseg;            // row mode: columns per item, column segments per row
     int32_t ra, nra;              // row mode: rows per item, row chunks per plane
-    int32_t tiled;                // 1: 32x32 tiles staged through shared memory
-    int32_t nta, ntb;             // tiled mode: tiles along the rows and the columns
+    int32_t tiled;                // 0 row mode, 1 tiles staged through shared memory, 2 direct transposing mode
+    int32_t nta, ntb;             // tiled and direct mode: tiles along the rows and the columns
 };
 
 struct DTerm {
@@ -416,9 +417,10 @@ cudaError_t launch_scatter_groups_dest(const DCrtComp *comps, const int64_t *res
 // Element-wise transfer kernels.  max_terms bounds nterms and tile_bytes the
 // shared-memory tiles of any tiled-mode job.
 // Units are ordered row-mode units first (nrow of them), then tiled-mode
-// units (ntiled); the dot product leaves one partial sum per unit.
+// units (ntiled), then direct-mode units (ndirect); the dot product (row and
+// tiled mode) leaves one partial sum per unit.
 cudaError_t launch_transfer(const DJob *jobs, const DTerm *terms, const DUnit *units,
-    int32_t nrow, int32_t ntiled, int32_t max_terms, int32_t tile_bytes, const double *const *srcs,
+    int32_t nrow, int32_t ntiled, int32_t ndirect, int32_t max_terms, int32_t tile_bytes, const double *const *srcs,
     double *dst, int32_t accumulate, double beta, cudaStream_t s);
 cudaError_t launch_dot(const DJob *jobs, const DTerm *terms, const DUnit *units,
     int32_t nrow, int32_t ntiled, int32_t tile_bytes, const double *a, const double *b,
