@@ -31,13 +31,13 @@ namespace {
 __device__ __forceinline__ int64_t mixed_offset(int32_t lin, int n, const int32_t *ext,
                                                 const int32_t *str) {
     int64_t off = 0;
-    for (int i = n - 1; i >= 0; i--) {
+    for (int i = n - 1; i > 0; i--) {
         int32_t e = ext[i];
         int32_t q = lin / e;
         off += (int64_t)(lin - q * e) * str[i];
         lin = q;
     }
-    return off;
+    return n > 0 ? off + (int64_t)lin * str[0] : off;      // the outermost digit is what is left
 }
 
 __device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool pred) {
@@ -97,7 +97,7 @@ struct TileCfg {
     static constexpr int kMT = WM / kFragRows, kNT = WN / 8;
     static constexpr int kStageA = BM * kLd, kStageB = BN * kLd;
     static constexpr size_t kSmem = (size_t)STAGES * (kStageA + kStageB) * sizeof(double)
-                                  + (size_t)(BM + BN) * sizeof(int64_t);
+                                  + (size_t)(BM + BN) * (sizeof(int64_t) + sizeof(int2));
     static_assert(kThreads % BK == 0 && kThreads % (BK / 2) == 0, "loader assumes a fixed k column per thread");
     static_assert(BM % WM == 0 && BN % WN == 0 && WM % kFragRows == 0 && WN % 8 == 0, "warp tiling");
     static_assert(BK % 8 == 0, "k step");
@@ -150,6 +150,9 @@ __device__ __forceinline__ void load_stage(double *sA, double *sB, const int64_t
     load_operand<C, C::BN>(sB, rowB, B, k0, t.K, t.nk, t.kext, t.kb_str, t.vec_b != 0);
 }
 
+// A work item is a tile of a stack of C blocks (DStack): rows of several blocks
+// share a tile where the blocks' products share their operands, so that blocks
+// of a few dozen rows fill whole tiles.
 // SCATTER: the epilogue writes each C block's tile to the destinations
 // dests[drange[cblk].x .. drange[cblk].y) instead of the block itself --
 // blocks of another tensor, each through its own index mapping and scale
@@ -158,6 +161,7 @@ __device__ __forceinline__ void load_stage(double *sA, double *sB, const int64_t
 template<class C, bool SCATTER>
 __global__ void __launch_bounds__(C::kThreads, C::MINB)
 contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict__ cblks,
+                     const DStack *__restrict__ stacks, const int32_t *__restrict__ stab,
                      const DItem *__restrict__ items, int32_t nitems, int32_t *counter,
                      const double *__restrict__ A, const double *__restrict__ B,
                      double *__restrict__ Cp, double *__restrict__ ws, int32_t add,
@@ -167,6 +171,7 @@ contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict_
     double *sB = smem + C::STAGES * C::kStageA;
     int64_t *rowA = reinterpret_cast<int64_t *>(sB + C::STAGES * C::kStageB);
     int64_t *rowB = rowA + C::BM;
+    int2 *rowinfo = reinterpret_cast<int2 *>(rowB + C::BN);     // tile rows, then columns: first task of the block, index in it
     __shared__ int32_t s_item;
     __shared__ __align__(16) DTask s_task;
 
@@ -182,8 +187,30 @@ contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict_
         __syncthreads();
         if (it >= nitems) break;
         const DItem item = items[it];
-        const DCBlock &cb = cblks[item.cblk];
-        const int M = cb.M, N = cb.N;
+        const DStack sk = stacks[item.stack];
+        const int32_t *rs = stab + sk.r0, *ss = stab + sk.s0, *grid = stab + sk.g0;
+        const int t_begin = cblks[grid[0]].t_begin, ntask = cblks[grid[0]].t_end - t_begin;
+        // each row (column) by the thread that will offset it
+        for (int r = tid; r < C::BM; r += C::kThreads) {
+            const int m = item.m0 + r;
+            int2 x = make_int2(-1, 0);
+            if (m < sk.M) {
+                int R = 0;
+                while (m >= rs[R + 1]) R++;
+                x = make_int2(cblks[grid[R * sk.ns]].t_begin, m - rs[R]);
+            }
+            rowinfo[r] = x;
+        }
+        for (int r = tid; r < C::BN; r += C::kThreads) {
+            const int n = item.n0 + r;
+            int2 x = make_int2(-1, 0);
+            if (n < sk.N) {
+                int S = 0;
+                while (n >= ss[S + 1]) S++;
+                x = make_int2(cblks[grid[S]].t_begin, n - ss[S]);
+            }
+            rowinfo[C::BM + r] = x;
+        }
 
         // lane fragment q of tile (i, j): row i * kFragRows + g + 8 (q >> 1),
         // column j * 8 + 2 t4 + (q & 1) of the warp tile
@@ -196,9 +223,9 @@ contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict_
                 for (int q = 0; q < C::kQ; q++) acc[i][j][q] = 0.0;
 
         int kt_base = 0;                       // k tiles of the tasks before ti
-        for (int ti = cb.t_begin; ti < cb.t_end && kt_base < item.kt1; ti++) {
+        for (int ti = 0; ti < ntask && kt_base < item.kt1; ti++) {
             // this item's k tiles of the task (a k chunk may cover part of it)
-            const int nkt_task = (tasks[ti].K + C::BK - 1) / C::BK;
+            const int nkt_task = (tasks[t_begin + ti].K + C::BK - 1) / C::BK;
             const int kt_lo = max(item.kt0 - kt_base, 0);
             const int kt_hi = min(item.kt1 - kt_base, nkt_task);
             kt_base += nkt_task;
@@ -206,16 +233,26 @@ contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict_
             static_assert(sizeof(DTask) % 8 == 0, "task copy granularity");
             if (tid < (int)(sizeof(DTask) / 8))
                 reinterpret_cast<int64_t *>(&s_task)[tid] =
-                    reinterpret_cast<const int64_t *>(&tasks[ti])[tid];
+                    reinterpret_cast<const int64_t *>(&tasks[t_begin + ti])[tid];
             __syncthreads();
             const DTask &t = s_task;
             for (int r = tid; r < C::BM; r += C::kThreads) {
-                int m = item.m0 + r;
-                rowA[r] = m < M ? t.a_off + mixed_offset(m, t.nm, t.mext, t.ma_str) : -1;
+                const int2 x = rowinfo[r];
+                int64_t off = -1;
+                if (x.x >= 0) {
+                    const DTask &u = tasks[x.x + ti];
+                    off = u.a_off + mixed_offset(x.y, u.nm, u.mext, u.ma_str);
+                }
+                rowA[r] = off;
             }
             for (int r = tid; r < C::BN; r += C::kThreads) {
-                int n = item.n0 + r;
-                rowB[r] = n < N ? t.b_off + mixed_offset(n, t.nn, t.next, t.nb_str) : -1;
+                const int2 x = rowinfo[C::BM + r];
+                int64_t off = -1;
+                if (x.x >= 0) {
+                    const DTask &u = tasks[x.x + ti];
+                    off = u.b_off + mixed_offset(x.y, u.nn, u.next, u.nb_str);
+                }
+                rowB[r] = off;
             }
             __syncthreads();
             const double coef = t.coeff;
@@ -342,73 +379,60 @@ contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict_
             continue;
         }
 
-        if constexpr (SCATTER) {
-            const int2 dr = drange[item.cblk];
-            for (int d = dr.x; d < dr.y; d++) {
-                const DCBlock &db = dests[d];
-                int64_t dm[C::kMT][C::kQ / 2];
-                int64_t dn[C::kNT][2];
+        // the tile's part of each C block it covers (one, unless blocks of the
+        // stack meet inside it)
+        for (int R = 0; R < sk.nr; R++) {
+            if (rs[R + 1] <= item.m0 || rs[R] >= item.m0 + C::BM) continue;
+            for (int S = 0; S < sk.ns; S++) {
+                if (ss[S + 1] <= item.n0 || ss[S] >= item.n0 + C::BN) continue;
+                const int cblk = grid[R * sk.ns + S];
+                const DCBlock &cb = cblks[cblk];
+                // first tile row and column in the block's own numbering
+                const int mb = item.m0 + wm * C::WM + g - rs[R], nb = item.n0 + wn * C::WN + 2 * t4 - ss[S];
+                // SCATTER: the block's destinations; else the block itself,
+                // scaled store (assign) or scaled accumulate (add)
+                int d0 = 0, d1 = 1;
+                if constexpr (SCATTER) {
+                    const int2 dr = drange[cblk];
+                    d0 = dr.x;
+                    d1 = dr.y;
+                }
+                for (int d = d0; d < d1; d++) {
+                    const DCBlock &db = SCATTER ? dests[d] : cb;
+                    const double scale = db.scale;
+                    int64_t dm[C::kMT][C::kQ / 2];
+                    int64_t dn[C::kNT][2];
 #pragma unroll
-                for (int i = 0; i < C::kMT; i++)
+                    for (int i = 0; i < C::kMT; i++)
 #pragma unroll
-                    for (int h = 0; h < C::kQ / 2; h++) {
-                        int m = item.m0 + wm * C::WM + i * C::kFragRows + g + 8 * h;
-                        dm[i][h] = m < M ? mixed_offset(m, db.nm, db.mext, db.mc_str) : -1;
-                    }
-#pragma unroll
-                for (int j = 0; j < C::kNT; j++)
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        int n = item.n0 + wn * C::WN + j * 8 + 2 * t4 + h;
-                        dn[j][h] = n < N ? mixed_offset(n, db.nn, db.next, db.nc_str) : -1;
-                    }
-                double *Db = Cp + db.c_off;
-#pragma unroll
-                for (int i = 0; i < C::kMT; i++)
+                        for (int h = 0; h < C::kQ / 2; h++) {
+                            const int m = mb + i * C::kFragRows + 8 * h;
+                            dm[i][h] = m >= 0 && m < cb.M ? mixed_offset(m, db.nm, db.mext, db.mc_str) : -1;
+                        }
 #pragma unroll
                     for (int j = 0; j < C::kNT; j++)
 #pragma unroll
-                        for (int q = 0; q < C::kQ; q++) {
-                            int64_t om = dm[i][q >> 1], on = dn[j][q & 1];
-                            if (om < 0 || on < 0) continue;
-                            atomicAdd(Db + om + on, db.scale * acc[i][j][q]);
+                        for (int h = 0; h < 2; h++) {
+                            const int n = nb + j * 8 + h;
+                            dn[j][h] = n >= 0 && n < cb.N ? mixed_offset(n, db.nn, db.next, db.nc_str) : -1;
                         }
-            }
-            continue;
-        }
-
-        // Epilogue: scaled store (assign) or scaled accumulate (add) into the
-        // canonical C block through its own index mapping.
-        const double scale = cb.scale;
-        int64_t coff_m[C::kMT][C::kQ / 2];
-        int64_t coff_n[C::kNT][2];
+                    double *Db = Cp + db.c_off;
 #pragma unroll
-        for (int i = 0; i < C::kMT; i++)
+                    for (int i = 0; i < C::kMT; i++)
 #pragma unroll
-            for (int h = 0; h < C::kQ / 2; h++) {
-                int m = item.m0 + wm * C::WM + i * C::kFragRows + g + 8 * h;
-                coff_m[i][h] = m < M ? mixed_offset(m, cb.nm, cb.mext, cb.mc_str) : -1;
-            }
+                        for (int j = 0; j < C::kNT; j++)
 #pragma unroll
-        for (int j = 0; j < C::kNT; j++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                int n = item.n0 + wn * C::WN + j * 8 + 2 * t4 + h;
-                coff_n[j][h] = n < N ? mixed_offset(n, cb.nn, cb.next, cb.nc_str) : -1;
-            }
-        double *Cb = Cp + cb.c_off;
-#pragma unroll
-        for (int i = 0; i < C::kMT; i++)
-#pragma unroll
-            for (int j = 0; j < C::kNT; j++)
-#pragma unroll
-                for (int q = 0; q < C::kQ; q++) {
-                    int64_t om = coff_m[i][q >> 1], on = coff_n[j][q & 1];
-                    if (om < 0 || on < 0) continue;
-                    double v = scale * acc[i][j][q];
-                    if (add) Cb[om + on] += v;
-                    else Cb[om + on] = v;
+                            for (int q = 0; q < C::kQ; q++) {
+                                const int64_t om = dm[i][q >> 1], on = dn[j][q & 1];
+                                if (om < 0 || on < 0) continue;
+                                const double v = scale * acc[i][j][q];
+                                if constexpr (SCATTER) atomicAdd(Db + om + on, v);
+                                else if (add) Db[om + on] += v;
+                                else Db[om + on] = v;
+                            }
                 }
+            }
+        }
     }
 }
 
@@ -416,6 +440,7 @@ contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict_
 // (fixed order: the result does not depend on which CTA ran which chunk).
 __global__ void __launch_bounds__(256)
 split_reduce_kernel(const DSplit *__restrict__ splits, int32_t nsplits, const DCBlock *__restrict__ cblks,
+                    const DStack *__restrict__ stacks, const int32_t *__restrict__ stab,
                     const double *__restrict__ ws, int32_t bm, int32_t bn, double *__restrict__ Cp,
                     int32_t add) {
     const int64_t tile = (int64_t)bm * bn;
@@ -426,9 +451,15 @@ split_reduce_kernel(const DSplit *__restrict__ splits, int32_t nsplits, const DC
         const int32_t r = (int32_t)((e - (int64_t)x * tile) / bn);
         const int32_t cc = (int32_t)(e - (int64_t)x * tile - (int64_t)r * bn);
         const DSplit sp = splits[x];
-        const DCBlock &cb = cblks[sp.cblk];
-        const int m = sp.m0 + r, n = sp.n0 + cc;
-        if (m >= cb.M || n >= cb.N) continue;
+        const DStack sk = stacks[sp.stack];
+        int m = sp.m0 + r, n = sp.n0 + cc;
+        if (m >= sk.M || n >= sk.N) continue;
+        int R = 0, S = 0;
+        while (m >= stab[sk.r0 + R + 1]) R++;
+        while (n >= stab[sk.s0 + S + 1]) S++;
+        m -= stab[sk.r0 + R];
+        n -= stab[sk.s0 + S];
+        const DCBlock &cb = cblks[stab[sk.g0 + R * sk.ns + S]];
         const double *p = ws + (int64_t)sp.slot0 * tile + (int64_t)r * bn + cc;
         double v = 0.0;
         for (int q = 0; q < sp.nparts; q++) v += p[(int64_t)q * tile];
@@ -441,7 +472,7 @@ split_reduce_kernel(const DSplit *__restrict__ splits, int32_t nsplits, const DC
 }
 
 template<class C, bool SCATTER>
-cudaError_t launch_cfg_s(const DTask *tasks, const DCBlock *cblks, const DItem *items,
+cudaError_t launch_cfg_s(const DTask *tasks, const DCBlock *cblks, const DStack *stacks, const int32_t *stab, const DItem *items,
                          int32_t nitems, int32_t *counter, const double *a, const double *b,
                          double *c, double *ws, int32_t add, const int2 *drange, const DCBlock *dests,
                          cudaStream_t s) {
@@ -460,19 +491,19 @@ cudaError_t launch_cfg_s(const DTask *tasks, const DCBlock *cblks, const DItem *
     if (grid < 1) return cudaSuccess;
     e = cudaMemsetAsync(counter, 0, sizeof(int32_t), s);
     if (e != cudaSuccess) return e;
-    contract_fp64_kernel<C, SCATTER><<<grid, C::kThreads, C::kSmem, s>>>(tasks, cblks, items, nitems, counter,
+    contract_fp64_kernel<C, SCATTER><<<grid, C::kThreads, C::kSmem, s>>>(tasks, cblks, stacks, stab, items, nitems, counter,
                                                                         a, b, c, ws, add, drange, dests);
     return cudaGetLastError();
 }
 
 template<class C>
-cudaError_t launch_cfg(const DTask *tasks, const DCBlock *cblks, const DItem *items,
+cudaError_t launch_cfg(const DTask *tasks, const DCBlock *cblks, const DStack *stacks, const int32_t *stab, const DItem *items,
                        int32_t nitems, int32_t *counter, const double *a, const double *b,
                        double *c, double *ws, int32_t add, const int2 *drange, const DCBlock *dests,
                        cudaStream_t s) {
     if (dests)
-        return launch_cfg_s<C, true>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    return launch_cfg_s<C, false>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, nullptr, nullptr, s);
+        return launch_cfg_s<C, true>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    return launch_cfg_s<C, false>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, nullptr, nullptr, s);
 }
 
 // Tile configurations (BM, BN, BK, warp tile M, warp tile N, stages).
@@ -525,7 +556,7 @@ int tile_cfg_bn(int cfg) {
 }
 
 cudaError_t launch_split_reduce(const DSplit *splits, int32_t nsplits, const DCBlock *cblks,
-    const double *ws, int32_t bm, int32_t bn, double *c, int32_t add, cudaStream_t s) {
+    const DStack *stacks, const int32_t *stab, const double *ws, int32_t bm, int32_t bn, double *c, int32_t add, cudaStream_t s) {
     if (nsplits <= 0) return cudaSuccess;
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
@@ -539,37 +570,37 @@ cudaError_t launch_split_reduce(const DSplit *splits, int32_t nsplits, const DCB
         return n;
     }();
     const int grid = (int)(want < (int64_t)per_sm * nsm ? want : (int64_t)per_sm * nsm);
-    split_reduce_kernel<<<grid, 256, 0, s>>>(splits, nsplits, cblks, ws, bm, bn, c, add);
+    split_reduce_kernel<<<grid, 256, 0, s>>>(splits, nsplits, cblks, stacks, stab, ws, bm, bn, c, add);
     return cudaGetLastError();
 }
 
-cudaError_t launch_contract_fp64(const DTask *tasks, const DCBlock *cblks,
-    const DItem *items, int32_t nitems, int32_t *counter, const double *a,
+cudaError_t launch_contract_fp64(const DTask *tasks, const DCBlock *cblks, const DStack *stacks,
+    const int32_t *stab, const DItem *items, int32_t nitems, int32_t *counter, const double *a,
     const double *b, double *c, double *ws, int32_t add, int32_t tile_cfg, cudaStream_t s,
     const int2 *drange, const DCBlock *dests) {
     switch (tile_cfg) {
-    case 0: return launch_cfg<Cfg0>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 1: return launch_cfg<Cfg1>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 2: return launch_cfg<Cfg2>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 3: return launch_cfg<Cfg3>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 4: return launch_cfg<Cfg4>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 5: return launch_cfg<Cfg5>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 6: return launch_cfg<Cfg6>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 7: return launch_cfg<Cfg7>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 8: return launch_cfg<Cfg8>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 9: return launch_cfg<Cfg9>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 10: return launch_cfg<Cfg10>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 11: return launch_cfg<Cfg11>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 12: return launch_cfg<Cfg12>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 13: return launch_cfg<Cfg13>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 14: return launch_cfg<Cfg14>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 15: return launch_cfg<Cfg15>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 16: return launch_cfg<Cfg16>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 17: return launch_cfg<Cfg17>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 18: return launch_cfg<Cfg18>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 19: return launch_cfg<Cfg19>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    case 20: return launch_cfg<Cfg20>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
-    default: return launch_cfg<Cfg21>(tasks, cblks, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 0: return launch_cfg<Cfg0>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 1: return launch_cfg<Cfg1>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 2: return launch_cfg<Cfg2>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 3: return launch_cfg<Cfg3>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 4: return launch_cfg<Cfg4>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 5: return launch_cfg<Cfg5>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 6: return launch_cfg<Cfg6>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 7: return launch_cfg<Cfg7>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 8: return launch_cfg<Cfg8>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 9: return launch_cfg<Cfg9>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 10: return launch_cfg<Cfg10>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 11: return launch_cfg<Cfg11>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 12: return launch_cfg<Cfg12>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 13: return launch_cfg<Cfg13>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 14: return launch_cfg<Cfg14>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 15: return launch_cfg<Cfg15>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 16: return launch_cfg<Cfg16>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 17: return launch_cfg<Cfg17>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 18: return launch_cfg<Cfg18>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 19: return launch_cfg<Cfg19>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    case 20: return launch_cfg<Cfg20>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
+    default: return launch_cfg<Cfg21>(tasks, cblks, stacks, stab, items, nitems, counter, a, b, c, ws, add, drange, dests, s);
     }
 }
 

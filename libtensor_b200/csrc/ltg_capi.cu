@@ -89,6 +89,28 @@ void upload_vec(DevBuf &d, const std::vector<T> &v, cudaStream_t s) {
     }
 }
 
+// Arrays of one plan in one device buffer: one allocation and one copy instead of
+// one each per array.
+struct DevPart {
+    void *p = nullptr;
+    template<class T> T *as() const { return static_cast<T *>(p); }
+};
+struct DevPack {
+    std::vector<char> bytes;
+    std::vector<std::pair<DevPart *, size_t>> parts;
+    template<class T>
+    void put(DevPart &part, const std::vector<T> &v) {
+        bytes.resize((bytes.size() + 255) / 256 * 256);
+        parts.push_back({&part, bytes.size()});
+        const char *p = reinterpret_cast<const char *>(v.data());
+        bytes.insert(bytes.end(), p, p + v.size() * sizeof(T));
+    }
+    void upload(DevBuf &d, cudaStream_t s) {
+        upload_vec(d, bytes, s);
+        for (auto &x : parts) x.first->p = static_cast<char *>(d.p) + x.second;
+    }
+};
+
 }  // namespace
 
 namespace ltg {
@@ -115,6 +137,22 @@ struct ltg_ctx {
     int nsm = 148;
     DevBuf scratch_counter;      // work-queue counters of persistent launches
     DevBuf dot_out;              // device scalar for synchronous dot products
+    // Workspace of the k-split partial tiles, one for all plans: every launch that
+    // fills it and the reduction that reads it follow each other on the context's
+    // stream.  It only grows, at least twofold; outgrown buffers stay until the
+    // context goes (plans and captured graphs point into them), so that all of
+    // them together are at most twice the largest.
+    std::vector<std::unique_ptr<DevBuf>> split_ws;
+    double *split_workspace(int64_t elems) {
+        const size_t need = (size_t)std::max<int64_t>(elems, 0) * sizeof(double);
+        if (need == 0) return nullptr;
+        if (split_ws.empty() || split_ws.back()->bytes < need) {
+            std::unique_ptr<DevBuf> b(new DevBuf());
+            b->alloc(std::max(need, split_ws.empty() ? (size_t)4 << 20 : 2 * split_ws.back()->bytes));
+            split_ws.push_back(std::move(b));
+        }
+        return split_ws.back()->as<double>();
+    }
     KernelTiming timing;
     // Bounded device waits of the tcgen05 kernels: the limit of one pipeline
     // wait, and the error word a kernel sets when a wait gave up (copied to
@@ -157,13 +195,16 @@ struct PlainGroups {
     int32_t ngroups = 0, nunits = 0, nsunits = 0;
     double scale = 1.0;                       // ka kb kc (and d in add mode)
     DevBuf buf, pieces, units, sunits, comps, res_off, ctab, cells;
-    DevBuf tasks, cblks, items, splits, ws;   // DMMA work over buf
+    DevBuf tasks, cblks, stacks, stab, items, splits;   // DMMA work over buf
+    double *ws = nullptr;                     // in the context's split workspace
     std::vector<DmmaLaunch> launches;
 };
 
 struct ContractExec {
     // device task arrays bound to one output tensor and coefficient set
-    DevBuf tasks, cblks, items, splits, ws;
+    DevBuf pack;
+    double *ws = nullptr;                     // in the context's split workspace
+    DevPart tasks, cblks, stacks, stab, items, splits;
     std::unique_ptr<PlainGroups> groups;      // grouped small blocks, if any
     std::vector<DmmaLaunch> launches;
     std::vector<std::pair<int64_t, int64_t>> zero_ranges;  // assign mode: blocks not in the schedule
@@ -176,7 +217,7 @@ struct ContractExec {
 // canonical blocks that take a term of the block, each with the term's index
 // mapping and sign), added atomically into the zeroed result.
 struct SymExec {
-    DevBuf tasks, cblks, items, drange, dests;
+    DevBuf tasks, cblks, stacks, stab, items, drange, dests;
     std::vector<DmmaLaunch> launches;
     // small blocks as the plain path's grouped products, their results
     // scattered from the group buffer to each cell's destinations
@@ -510,6 +551,106 @@ int pick_tile(int64_t M, int64_t N) {
     return best;
 }
 
+// Stacks of C blocks (DStack) and their table.
+struct PlainStacks {
+    std::vector<DStack> stacks;
+    std::vector<int32_t> tab;
+    int32_t first_block(int32_t stack) const { return tab[stacks[stack].g0]; }
+    // row and column blocks by representatives: rows (R, 0), columns (0, S)
+    void add(const std::vector<DCBlock> &dc, int32_t nr, int32_t ns, const std::vector<int32_t> &grid) {
+        DStack k{};
+        k.nr = nr; k.ns = ns;
+        k.r0 = (int32_t)tab.size();
+        for (int32_t R = 0; R < nr; R++) { tab.push_back(k.M); k.M += dc[grid[(size_t)R * ns]].M; }
+        tab.push_back(k.M);
+        k.s0 = (int32_t)tab.size();
+        for (int32_t S = 0; S < ns; S++) { tab.push_back(k.N); k.N += dc[grid[S]].N; }
+        tab.push_back(k.N);
+        k.g0 = (int32_t)tab.size();
+        tab.insert(tab.end(), grid.begin(), grid.end());
+        stacks.push_back(k);
+    }
+};
+
+// Stacks the C blocks e with use[e] != 0.  Blocks are linked when their products
+// read, task by task, the same rows of A or the same columns of B, with the same
+// k mapping, coefficient and load width; a linked set that fills its grid of
+// distinct A parts and B parts is one stack, else each of its columns is.
+// A ladder's occupied-pair blocks share every V block: ij blocks of 36, 42 and 49
+// rows fill 64-row tiles to 66 %, stacked (127 and 169 rows) to 93 %
+// (o=26 v=130 in blocks of 7, 6 and 29, 23, 13: 917 to 518 us with the cheaper epilogue).
+void plain_stacks(const std::vector<DTask> &dt, const std::vector<DCBlock> &dc, const std::vector<char> &use,
+                  PlainStacks &ps) {
+    auto put = [](std::string &k, const void *p, size_t n) { k.append(static_cast<const char *>(p), n); };
+    std::map<std::string, int32_t> ids;
+    std::vector<int32_t> up;
+    auto node = [&](std::string key) {
+        auto f = ids.emplace(std::move(key), (int32_t)up.size());
+        if (f.second) up.push_back((int32_t)up.size());
+        return f.first->second;
+    };
+    auto root = [&](int32_t x) {
+        while (up[x] != x) { up[x] = up[up[x]]; x = up[x]; }
+        return x;
+    };
+    std::vector<int32_t> ra(dc.size(), -1), sb(dc.size(), -1);
+    for (size_t e = 0; e < dc.size(); e++) {
+        if (!use[e]) continue;
+        std::string common, a = "a", b = "b";
+        put(a, &dc[e].M, sizeof(dc[e].M));
+        put(b, &dc[e].N, sizeof(dc[e].N));
+        for (int32_t i = dc[e].t_begin; i < dc[e].t_end; i++) {
+            const DTask &t = dt[i];
+            put(common, &t.coeff, sizeof(t.coeff));
+            put(common, &t.K, sizeof(t.K)); put(common, &t.nk, sizeof(t.nk));
+            put(common, t.kext, sizeof(t.kext)); put(common, t.ka_str, sizeof(t.ka_str)); put(common, t.kb_str, sizeof(t.kb_str));
+            put(common, &t.vec_a, sizeof(t.vec_a)); put(common, &t.vec_b, sizeof(t.vec_b));
+            put(a, &t.a_off, sizeof(t.a_off)); put(a, &t.nm, sizeof(t.nm));
+            put(a, t.mext, sizeof(t.mext)); put(a, t.ma_str, sizeof(t.ma_str));
+            put(b, &t.b_off, sizeof(t.b_off)); put(b, &t.nn, sizeof(t.nn));
+            put(b, t.next, sizeof(t.next)); put(b, t.nb_str, sizeof(t.nb_str));
+        }
+        ra[e] = node(a + common);
+        sb[e] = node(b + common);
+        const int32_t x = root(ra[e]), y = root(sb[e]);
+        if (x != y) up[x] = y;
+    }
+    std::map<int32_t, std::vector<int32_t>> sets;
+    for (size_t e = 0; e < dc.size(); e++)
+        if (use[e]) sets[root(ra[e])].push_back((int32_t)e);
+    std::vector<std::pair<int32_t, const std::vector<int32_t> *>> order;      // by first block
+    for (const auto &x : sets) order.push_back({x.second.front(), &x.second});
+    std::sort(order.begin(), order.end());
+    for (const auto &x : order) {
+        const std::vector<int32_t> &blocks = *x.second;
+        std::map<int32_t, int32_t> rows, cols;
+        int64_t M = 0, N = 0;
+        for (int32_t e : blocks) {
+            if (rows.emplace(ra[e], (int32_t)rows.size()).second) M += dc[e].M;
+            if (cols.emplace(sb[e], (int32_t)cols.size()).second) N += dc[e].N;
+        }
+        const bool fits = M < ((int64_t)1 << 30) && N < ((int64_t)1 << 30);
+        if (fits && rows.size() * cols.size() == blocks.size()) {
+            std::vector<int32_t> grid(blocks.size(), -1);
+            for (int32_t e : blocks) grid[(size_t)rows[ra[e]] * cols.size() + cols[sb[e]]] = e;
+            // (two blocks with equal products cannot both sit in one cell)
+            if (std::find(grid.begin(), grid.end(), -1) == grid.end()) {
+                ps.add(dc, (int32_t)rows.size(), (int32_t)cols.size(), grid);
+                continue;
+            }
+        }
+        std::map<int32_t, std::vector<int32_t>> by_col;
+        for (int32_t e : blocks) by_col[cols[sb[e]]].push_back(e);
+        for (const auto &c : by_col) {
+            if (fits) {
+                ps.add(dc, (int32_t)c.second.size(), 1, c.second);
+            } else {
+                for (int32_t e : c.second) ps.add(dc, 1, 1, {e});
+            }
+        }
+    }
+}
+
 // Work items of one tile shape, appended to `items` costliest first (LPT
 // order for the persistent work queue).  The tail of a launch is uneven when
 // its items are few and long; cutting the k range of the last items into
@@ -521,7 +662,7 @@ int pick_tile(int64_t M, int64_t N) {
 // work-queue order) at the nominal per-SM DMMA rate, plus the partial tiles'
 // bytes at HBM speed; 1 never splits; 2-4 split every item in that many.
 void append_launch(int cfg, std::vector<std::pair<double, DItem>> &v, const std::vector<DTask> &dt,
-                   const std::vector<DCBlock> &dc, int nsm, int split_k, std::vector<DItem> &items,
+                   const std::vector<DCBlock> &dc, const PlainStacks &ps, int nsm, int split_k, std::vector<DItem> &items,
                    std::vector<DSplit> &splits, int64_t &ws_elems, std::vector<DmmaLaunch> &launches) {
     if (v.empty()) return;
     std::stable_sort(v.begin(), v.end(), [](const std::pair<double, DItem> &x, const std::pair<double, DItem> &y) {
@@ -531,7 +672,7 @@ void append_launch(int cfg, std::vector<std::pair<double, DItem>> &v, const std:
     const size_t n = v.size();
     std::vector<int32_t> nkt(n, 0);
     for (size_t i = 0; i < n; i++) {
-        const DCBlock &b = dc[v[i].second.cblk];
+        const DCBlock &b = dc[ps.first_block(v[i].second.stack)];
         for (int32_t t = b.t_begin; t < b.t_end; t++) nkt[i] += (dt[t].K + bk - 1) / bk;
     }
     const double kFmaPerSmSec = 40e12 / 2 / 148, kBytesPerSec = 6e12, kReduceLaunchSec = 4e-6;
@@ -580,7 +721,7 @@ void append_launch(int cfg, std::vector<std::pair<double, DItem>> &v, const std:
         const int parts = i >= first_split ? std::max(1, std::min(sk, nkt[i])) : 1;
         if (parts == 1) { out.push_back(v[i]); continue; }
         DSplit sp;
-        sp.cblk = v[i].second.cblk; sp.m0 = v[i].second.m0; sp.n0 = v[i].second.n0;
+        sp.stack = v[i].second.stack; sp.m0 = v[i].second.m0; sp.n0 = v[i].second.n0;
         sp.nparts = parts; sp.slot0 = slot; sp.pad = 0;
         splits.push_back(sp);
         for (int p = 0; p < parts; p++) {
@@ -680,6 +821,25 @@ void plain_task_arrays(const ltg_plan *pl, int64_t c_elems, const std::vector<Ge
     }
 }
 
+// Work items of the stacks by tile shape: the plan's forced or autotuned shape,
+// or pick_tile's.
+void stack_items(const ltg_plan *pl, const PlainStacks &ps, const std::vector<CBlockTask> &cbt,
+                 std::vector<std::vector<std::pair<double, DItem>>> &per_cfg) {
+    for (size_t k = 0; k < ps.stacks.size(); k++) {
+        const DStack &st = ps.stacks[k];
+        const CBlockTask &b = cbt[ps.first_block((int32_t)k)];
+        int cfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(st.M, st.N);
+        auto ov = pl->tile_override.find({st.M, st.N});
+        if (pl->forced_tile < 0 && ov != pl->tile_override.end()) cfg = ov->second;
+        const int bm = tile_cfg_bm(cfg), bn = tile_cfg_bn(cfg);
+        for (int64_t m0 = 0; m0 < st.M; m0 += bm)
+            for (int64_t n0 = 0; n0 < st.N; n0 += bn) {
+                const double cost = (double)bm * bn * (b.kflops + 8.0 * (b.t_end - b.t_begin));
+                per_cfg[cfg].push_back({cost, make_item((int32_t)k, (int32_t)m0, (int32_t)n0)});
+            }
+    }
+}
+
 ContractExec *prepare_exec(ltg_plan *pl, ltg_bt *c, double ka, double kb, double kc, int add, double d) {
     auto key = std::make_tuple(c->uid, ka, kb, kc, add, add ? d : 0.0);
     auto it = pl->exec.find(key);
@@ -703,33 +863,28 @@ ContractExec *prepare_exec(ltg_plan *pl, ltg_bt *c, double ka, double kb, double
     }
     // Work items per tile configuration, costliest first (LPT order for the
     // persistent work queue).
+    std::vector<char> use(cbt.size(), 0);
+    for (size_t e = 0; e < cbt.size(); e++) use[e] = group_of[e] < 0;
+    PlainStacks ps;
+    plain_stacks(dt, dc, use, ps);
     std::vector<std::vector<std::pair<double, DItem>>> per_cfg(kNumShapes);
-    for (size_t e = 0; e < cbt.size(); e++) {
-        if (group_of[e] >= 0) continue;
-        int cfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(cbt[e].M, cbt[e].N);
-        auto ov = pl->tile_override.find({cbt[e].M, cbt[e].N});
-        if (pl->forced_tile < 0 && ov != pl->tile_override.end()) cfg = ov->second;
-        int bm = tile_cfg_bm(cfg), bn = tile_cfg_bn(cfg);
-        for (int64_t m0 = 0; m0 < cbt[e].M; m0 += bm)
-            for (int64_t n0 = 0; n0 < cbt[e].N; n0 += bn) {
-                DItem it = make_item((int32_t)e, (int32_t)m0, (int32_t)n0);
-                double cost = (double)bm * bn * (cbt[e].kflops + 8.0 * (cbt[e].t_end - cbt[e].t_begin));
-                per_cfg[cfg].push_back({cost, it});
-            }
-    }
+    stack_items(pl, ps, cbt, per_cfg);
     std::vector<DItem> items;
     std::vector<DSplit> splits;
     int64_t ws_elems = 0;
     for (int cfg = 0; cfg < kNumShapes; cfg++)
-        append_launch(cfg, per_cfg[cfg], dt, dc, pl->ctx->nsm, pl->split_k, items, splits, ws_elems, ex->launches);
+        append_launch(cfg, per_cfg[cfg], dt, dc, ps, pl->ctx->nsm, pl->split_k, items, splits, ws_elems, ex->launches);
     cudaStream_t s = pl->ctx->stream;
-    upload_vec(ex->tasks, dt, s);
-    upload_vec(ex->cblks, dc, s);
-    upload_vec(ex->items, items, s);
-    if (!splits.empty()) {
-        upload_vec(ex->splits, splits, s);
-        ex->ws.alloc(ws_elems * (int64_t)sizeof(double));
-    }
+    if (ps.stacks.empty()) { dt.clear(); dc.clear(); }        // all blocks grouped
+    DevPack pack;
+    pack.put(ex->tasks, dt);
+    pack.put(ex->cblks, dc);
+    pack.put(ex->items, items);
+    pack.put(ex->stacks, ps.stacks);
+    pack.put(ex->stab, ps.tab);
+    pack.put(ex->splits, splits);
+    pack.upload(ex->pack, s);
+    ex->ws = pl->ctx->split_workspace(ws_elems);
     // blocks of C outside the schedule (zeroed in assign mode)
     std::vector<char> in_sched(c->h.blk_abs.size(), 0);
     if (pl->external) {
@@ -1340,6 +1495,7 @@ void build_plain_groups(ltg_plan *pl, const BlockTensorHost &ch, const std::vect
     std::vector<DTask> dt;
     std::vector<DCBlock> dc;
     std::vector<std::vector<std::pair<double, DItem>>> per_cfg(kNumShapes);
+    PlainStacks ps;                           // stack g is group g's product
     int64_t off = 0;
     PlainGroupLayout lay;
     // one tile shape for all groups (one launch, one tail): that of the
@@ -1416,12 +1572,13 @@ void build_plain_groups(ltg_plan *pl, const BlockTensorHost &ch, const std::vect
                 per_cfg[cfg].push_back({(double)bm * bn * (double)lay.kt, it});
             }
         dc.push_back(b);
+        ps.add(dc, 1, 1, {(int32_t)dc.size() - 1});
     }
     std::vector<DItem> items;
     std::vector<DSplit> splits;
     int64_t ws_elems = 0;
     for (int cfg = 0; cfg < kNumShapes; cfg++)
-        append_launch(cfg, per_cfg[cfg], dt, dc, pl->ctx->nsm, pl->split_k, items, splits, ws_elems, pg.launches);
+        append_launch(cfg, per_cfg[cfg], dt, dc, ps, pl->ctx->nsm, pl->split_k, items, splits, ws_elems, pg.launches);
     cudaStream_t s = pl->ctx->stream;
     pg.ngroups = (int32_t)groups.size();
     pg.nunits = (int32_t)units.size();
@@ -1442,9 +1599,11 @@ void build_plain_groups(ltg_plan *pl, const BlockTensorHost &ch, const std::vect
     upload_vec(pg.tasks, dt, s);
     upload_vec(pg.cblks, dc, s);
     upload_vec(pg.items, items, s);
+    upload_vec(pg.stacks, ps.stacks, s);
+    upload_vec(pg.stab, ps.tab, s);
     if (!splits.empty()) {
         upload_vec(pg.splits, splits, s);
-        pg.ws.alloc(ws_elems * (int64_t)sizeof(double));
+        pg.ws = pl->ctx->split_workspace(ws_elems);
     }
 }
 
@@ -2842,31 +3001,25 @@ SymExec *prepare_sym(ltg_plan *pl, ltg_bt *r, int32_t mode, int32_t L, double c,
     }
     // work items of the other C blocks that reach the result, each over its
     // whole k range (tile shapes as in the plain path)
+    std::vector<char> use(cbt.size(), 0);
+    for (size_t e = 0; e < cbt.size() && !crt && !slice; e++) use[e] = !per[e].empty() && group_of[e] < 0;
+    PlainStacks ps;
+    plain_stacks(dt, dc, use, ps);
     std::vector<std::vector<std::pair<double, DItem>>> per_cfg(kNumShapes);
-    for (size_t e = 0; e < cbt.size() && !crt && !slice; e++) {
-        if (per[e].empty() || group_of[e] >= 0) continue;
-        int cfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(cbt[e].M, cbt[e].N);
-        auto ov = pl->tile_override.find({cbt[e].M, cbt[e].N});
-        if (pl->forced_tile < 0 && ov != pl->tile_override.end()) cfg = ov->second;
-        const int bm = tile_cfg_bm(cfg), bn = tile_cfg_bn(cfg);
-        for (int64_t m0 = 0; m0 < cbt[e].M; m0 += bm)
-            for (int64_t n0 = 0; n0 < cbt[e].N; n0 += bn) {
-                DItem di = make_item((int32_t)e, (int32_t)m0, (int32_t)n0);
-                const double cost = (double)bm * bn * (cbt[e].kflops + 8.0 * (cbt[e].t_end - cbt[e].t_begin));
-                per_cfg[cfg].push_back({cost, di});
-            }
-    }
+    stack_items(pl, ps, cbt, per_cfg);
     std::vector<DItem> items;
     std::vector<DSplit> splits;
     int64_t ws_elems = 0;
     for (int cfg = 0; cfg < kNumShapes; cfg++)
-        append_launch(cfg, per_cfg[cfg], dt, dc, pl->ctx->nsm, 1, items, splits, ws_elems, ex->launches);
+        append_launch(cfg, per_cfg[cfg], dt, dc, ps, pl->ctx->nsm, 1, items, splits, ws_elems, ex->launches);
     if (!splits.empty()) throw error(kErrState, "k chunks in a fused symmetrizer");
     if (dests.empty()) dests.resize(1);
     cudaStream_t s = pl->ctx->stream;
     upload_vec(ex->tasks, dt, s);
     upload_vec(ex->cblks, dc, s);
     upload_vec(ex->items, items, s);
+    upload_vec(ex->stacks, ps.stacks, s);
+    upload_vec(ex->stab, ps.tab, s);
     upload_vec(ex->drange, drange, s);
     upload_vec(ex->dests, dests, s);
     SymExec *raw = ex.get();
@@ -2981,14 +3134,15 @@ int ltg_contract2_symmetrized(ltg_plan *plan, ltg_bt *r, int32_t mode, int32_t n
             ctx->launches++;
             for (auto &l : pg->launches) {
                 TimedLaunch tl(ctx, LTG_KERNEL_CONTRACT_FP64);
-                LTG_CUDA(launch_contract_fp64(pg->tasks.as<DTask>(), pg->cblks.as<DCBlock>(),
+                LTG_CUDA(launch_contract_fp64(pg->tasks.as<DTask>(), pg->cblks.as<DCBlock>(), pg->stacks.as<DStack>(), pg->stab.as<int32_t>(),
                                               pg->items.as<DItem>() + l.item0, l.nitems,
                                               ctx->scratch_counter.as<int32_t>() + (slot++ % 64),
                                               pg->buf.as<double>(), pg->buf.as<double>(), pg->buf.as<double>(),
-                                              pg->ws.as<double>() + l.ws_off, 0, l.cfg, s));
+                                              pg->ws + l.ws_off, 0, l.cfg, s));
                 if (l.nsplits > 0) {
                     LTG_CUDA(launch_split_reduce(pg->splits.as<DSplit>() + l.split0, l.nsplits, pg->cblks.as<DCBlock>(),
-                                                 pg->ws.as<double>() + l.ws_off, tile_cfg_bm(l.cfg),
+                                                 pg->stacks.as<DStack>(), pg->stab.as<int32_t>(),
+                                                 pg->ws + l.ws_off, tile_cfg_bm(l.cfg),
                                                  tile_cfg_bn(l.cfg), pg->buf.as<double>(), 0, s));
                     ctx->launches++;
                 }
@@ -3006,7 +3160,7 @@ int ltg_contract2_symmetrized(ltg_plan *plan, ltg_bt *r, int32_t mode, int32_t n
         }
         for (auto &l : ex->launches) {
             TimedLaunch tl(ctx, LTG_KERNEL_CONTRACT_FP64);
-            LTG_CUDA(launch_contract_fp64(ex->tasks.as<DTask>(), ex->cblks.as<DCBlock>(),
+            LTG_CUDA(launch_contract_fp64(ex->tasks.as<DTask>(), ex->cblks.as<DCBlock>(), ex->stacks.as<DStack>(), ex->stab.as<int32_t>(),
                                           ex->items.as<DItem>() + l.item0, l.nitems,
                                           ctx->scratch_counter.as<int32_t>() + (slot++ % 64),
                                           plan->a->arena.as<double>(), plan->b->arena.as<double>(),
@@ -3540,14 +3694,15 @@ int ltg_contract2(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nslices, doub
             ctx->launches++;
             for (auto &l : pg->launches) {
                 TimedLaunch tl(ctx, LTG_KERNEL_CONTRACT_FP64);
-                LTG_CUDA(launch_contract_fp64(pg->tasks.as<DTask>(), pg->cblks.as<DCBlock>(),
+                LTG_CUDA(launch_contract_fp64(pg->tasks.as<DTask>(), pg->cblks.as<DCBlock>(), pg->stacks.as<DStack>(), pg->stab.as<int32_t>(),
                                               pg->items.as<DItem>() + l.item0, l.nitems,
                                               ctx->scratch_counter.as<int32_t>() + (slot++ % 64),
                                               pg->buf.as<double>(), pg->buf.as<double>(), pg->buf.as<double>(),
-                                              pg->ws.as<double>() + l.ws_off, 0, l.cfg, s));
+                                              pg->ws + l.ws_off, 0, l.cfg, s));
                 if (l.nsplits > 0) {
                     LTG_CUDA(launch_split_reduce(pg->splits.as<DSplit>() + l.split0, l.nsplits, pg->cblks.as<DCBlock>(),
-                                                 pg->ws.as<double>() + l.ws_off, tile_cfg_bm(l.cfg),
+                                                 pg->stacks.as<DStack>(), pg->stab.as<int32_t>(),
+                                                 pg->ws + l.ws_off, tile_cfg_bm(l.cfg),
                                                  tile_cfg_bn(l.cfg), pg->buf.as<double>(), 0, s));
                     ctx->launches++;
                 }
@@ -3557,14 +3712,15 @@ int ltg_contract2(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nslices, doub
         }
         for (auto &l : ex->launches) {
             TimedLaunch tl(ctx, LTG_KERNEL_CONTRACT_FP64);
-            LTG_CUDA(launch_contract_fp64(ex->tasks.as<DTask>(), ex->cblks.as<DCBlock>(),
+            LTG_CUDA(launch_contract_fp64(ex->tasks.as<DTask>(), ex->cblks.as<DCBlock>(), ex->stacks.as<DStack>(), ex->stab.as<int32_t>(),
                                           ex->items.as<DItem>() + l.item0, l.nitems,
                                           ctx->scratch_counter.as<int32_t>() + (slot++ % 64),
                                           plan->a->arena.as<double>(), plan->b->arena.as<double>(),
-                                          c->arena.as<double>(), ex->ws.as<double>() + l.ws_off, add, l.cfg, s));
+                                          c->arena.as<double>(), ex->ws + l.ws_off, add, l.cfg, s));
             if (l.nsplits > 0) {
                 LTG_CUDA(launch_split_reduce(ex->splits.as<DSplit>() + l.split0, l.nsplits, ex->cblks.as<DCBlock>(),
-                                             ex->ws.as<double>() + l.ws_off, tile_cfg_bm(l.cfg), tile_cfg_bn(l.cfg),
+                                                 ex->stacks.as<DStack>(), ex->stab.as<int32_t>(),
+                                             ex->ws + l.ws_off, tile_cfg_bm(l.cfg), tile_cfg_bn(l.cfg),
                                              c->arena.as<double>(), add, s));
                 ctx->launches++;
             }
@@ -3741,8 +3897,17 @@ int ltg_contract2_autotune(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nsli
             mode == LTG_MODE_PLAIN_FP64 ? plain_group_shapes(plan, c, cbt, group_of)
                                         : std::vector<std::pair<int64_t, int64_t>>();
         if (group_of.size() != cbt.size()) group_of.assign(cbt.size(), -1);
-        for (size_t e = 0; e < cbt.size(); e++)
-            if (group_of[e] < 0) work[{cbt[e].M, cbt[e].N}] += (double)cbt[e].M * cbt[e].N * cbt[e].kflops;
+        std::vector<DTask> dt;
+        std::vector<DCBlock> dc;
+        plain_task_arrays(plan, c->h.total_elems, tasks, cbt, 1.0, dt, dc);
+        std::vector<char> use(cbt.size(), 0);
+        for (size_t e = 0; e < cbt.size(); e++) use[e] = group_of[e] < 0;
+        PlainStacks ps;
+        plain_stacks(dt, dc, use, ps);
+        for (size_t k = 0; k < ps.stacks.size(); k++) {
+            const DStack &st = ps.stacks[k];
+            work[{st.M, st.N}] += (double)st.M * st.N * cbt[ps.first_block((int32_t)k)].kflops;
+        }
         for (const auto &g : gshapes) work[g] += (double)g.first * g.second;
         std::vector<std::pair<double, std::pair<int64_t, int64_t>>> order;
         for (auto &w : work) order.push_back({w.second, w.first});

@@ -37,13 +37,25 @@ struct DCBlock {
     int32_t t_begin, t_end;       // task range
 };
 
-// One CTA work item: an (m, n) tile of a C block, over the k tiles
-// [kt0, kt1) of the C block's task sequence (every task's k tiles in task
-// order).  slot < 0: the item covers all k tiles and writes C itself;
+// C blocks computed as one product: a grid of row blocks R and column blocks S
+// whose block (R, S) has, task by task, the A rows of (R, 0), the B columns of
+// (0, S) and the k mapping and relative coefficient of (0, 0).  Rows and columns
+// are numbered through the grid: tab[r0 + R] is the first row of row block R
+// (nr + 1 entries), tab[s0 + S] the first column of column block S, and
+// tab[g0 + R * ns + S] the C block.
+struct DStack {
+    int32_t M, N;
+    int32_t nr, ns;
+    int32_t r0, s0, g0;
+    int32_t pad;
+};
+
+// One CTA work item: an (m, n) tile of a stack, over the k tiles [kt0, kt1) of
+// its task sequence (every task's k tiles in task order).  slot < 0: the item covers all k tiles and writes C itself;
 // slot >= 0: a k chunk whose partial tile goes to workspace slot `slot`,
 // summed in chunk order by the split reduction.
 struct DItem {
-    int32_t cblk;
+    int32_t stack;
     int32_t m0, n0;
     int32_t slot;
     int32_t kt0, kt1;
@@ -52,16 +64,16 @@ struct DItem {
 // A tile whose k range was split into nparts chunks (workspace slots
 // slot0 .. slot0 + nparts - 1, in k order).
 struct DSplit {
-    int32_t cblk;
+    int32_t stack;
     int32_t m0, n0;
     int32_t nparts;
     int32_t slot0;
     int32_t pad;
 };
 
-inline DItem make_item(int32_t cblk, int32_t m0, int32_t n0) {
+inline DItem make_item(int32_t stack, int32_t m0, int32_t n0) {
     DItem it;
-    it.cblk = cblk; it.m0 = m0; it.n0 = n0;
+    it.stack = stack; it.m0 = m0; it.n0 = n0;
     it.slot = -1; it.kt0 = 0; it.kt1 = INT32_MAX;
     return it;
 }
@@ -309,14 +321,14 @@ __host__ __device__ inline double seeded_value(const DGenGroup &g, uint64_t seed
 // With dests (and drange, one index range of dests per C block), every C
 // block's tile is added atomically to its destinations instead of being
 // written (no k chunks: every item covers its whole k range).
-cudaError_t launch_contract_fp64(const DTask *tasks, const DCBlock *cblks,
-    const DItem *items, int32_t nitems, int32_t *counter, const double *a,
+cudaError_t launch_contract_fp64(const DTask *tasks, const DCBlock *cblks, const DStack *stacks,
+    const int32_t *stab, const DItem *items, int32_t nitems, int32_t *counter, const double *a,
     const double *b, double *c, double *ws, int32_t add, int32_t tile_cfg, cudaStream_t s,
     const int2 *drange = nullptr, const DCBlock *dests = nullptr);
 // Sums the partial tiles of every split tile in chunk order and writes (or
 // adds) the scaled result into its C block.
 cudaError_t launch_split_reduce(const DSplit *splits, int32_t nsplits, const DCBlock *cblks,
-    const double *ws, int32_t bm, int32_t bn, double *c, int32_t add, cudaStream_t s);
+    const DStack *stacks, const int32_t *stab, const double *ws, int32_t bm, int32_t bn, double *c, int32_t add, cudaStream_t s);
 int tile_cfg_bk(int cfg);
 
 // Split-precision contraction: FP64 -> slice tile images, then the tcgen05
