@@ -119,13 +119,13 @@ struct StaticFor<E, E> {
 
 __device__ __forceinline__ int64_t mixed_offset(int32_t lin, int n, const int32_t *ext, const int32_t *str) {
     int64_t off = 0;
-    for (int i = n - 1; i >= 0; i--) {
+    for (int i = n - 1; i > 0; i--) {
         const int32_t e = ext[i];
         const int32_t q = lin / e;
         off += (int64_t)(lin - q * e) * str[i];
         lin = q;
     }
-    return off;
+    return n > 0 ? off + (int64_t)lin * str[0] : off;      // the outermost digit is what is left
 }
 
 // Byte offset of element (row r, k byte kb_byte of k block kb) of modulus l
@@ -183,13 +183,39 @@ __device__ __forceinline__ int64_t koffset(const DCrtPanel &P, int mode, const i
     return mode == 0 ? k : (mode == 1 ? koff[k] : mixed_offset(k, P.nk, P.kext, P.kstr));
 }
 
-__global__ void __launch_bounds__(kSplitThreads)
+// Largest magnitude of a row as integers: the largest high word without its sign,
+// and all low words or'ed (their highest bit is that of the largest subnormal
+// below 2^-1042, whose high word is zero).  FP64 maxima and one load in flight
+// per thread held the pass to a quarter of the HBM rate (ladder o=20 v=90: 48 us
+// for 78 MB, 20 this way with two 32-byte groups in flight; more of them cost the
+// core tiles of short rows their occupancy; ring D2h 71 to 68 us).
+struct RowMax {
+    uint32_t hi = 0, lo = 0;
+    __device__ __forceinline__ void take(double x) {
+        hi = max(hi, (uint32_t)__double2hiint(x) & 0x7fffffffu);
+        lo |= (uint32_t)__double2loint(x);
+    }
+    __device__ __forceinline__ void join(int lanes) {
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, lanes));
+        lo |= __shfl_xor_sync(0xffffffffu, lo, lanes);
+    }
+    // e with |x| in [2^(e-1), 2^e), or kNoExp without a non-zero element
+    __device__ __forceinline__ int exponent() const {
+        if ((hi | lo) == 0) return kNoExp;
+        int e;
+        frexp(__hiloint2double((int)hi, (int)lo), &e);
+        return e;
+    }
+};
+
+__global__ void __launch_bounds__(kSplitThreads, 6)
 crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ units, int32_t nunits,
                const double *__restrict__ A, const double *__restrict__ B, const int32_t *__restrict__ gidx,
                int32_t *ex, int32_t *ey, int32_t sample) {
     __shared__ int32_t koff[kKoffMax];
     __shared__ int32_t rexp[kUnitRowsMax];
     __shared__ int64_t roff[kUnitRowsMax];                  // tile mapping: the unit's row offsets
+    constexpr int kAhead = 2;                               // 4-element groups in flight per thread
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lrow = lane >> 2, kq = lane & 3;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const int4 un = units[u];
@@ -203,11 +229,23 @@ crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
         if (un.w == kUnitTileMap)
             for (int i = threadIdx.x; i < un.z; i += blockDim.x) {
                 rexp[i] = kNoExp;
-                roff[i] = un.y + i < P.rows ? mixed_offset(un.y + i, P.nr, P.rext, P.rstr) : 0;
+                roff[i] = un.y + i < P.rows ? mixed_offset(un.y + i, P.nr, P.rext, P.rstr) : -1;
             }
         if (shared) __syncthreads();
         const double *src = (P.src ? B : A) + P.src_off;
         int32_t *tab = P.side == 0 ? ex : ey;
+        const int K = P.K;
+        // elements k0..k0+3 of a row, zero past K
+        auto load4 = [&](const double *row, int k0, double *x) {
+            if (mode == 0 && ((uintptr_t)row & 15) == 0 && k0 + 3 < K) {
+                const double2 a = *reinterpret_cast<const double2 *>(row + k0);
+                const double2 b = *reinterpret_cast<const double2 *>(row + k0 + 2);
+                x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+                return;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) x[j] = k0 + j < K ? row[koffset(P, mode, koff, k0 + j)] : 0.0;
+        };
         if (un.w == kUnitRowMap) {
             const int lr = threadIdx.x >> 3, c = threadIdx.x & 7;
             const int r = un.y + lr;
@@ -216,45 +254,53 @@ crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
             // sampled: group c of every kSampleGroups-th run of 32 elements;
             // else group c of every run
             const bool smp = sample && sampled_panel(P, un.w);
-            const int step = smp ? 32 * kSampleGroups : 32, first = 4 * c;
-            double mx = 0.0;
+            const int step = smp ? 32 * kSampleGroups : 32;
+            RowMax m;
             if (valid)
-                for (int k0 = first; k0 < P.K; k0 += step)
+                for (int k0 = 4 * c; k0 < K; k0 += kAhead * step) {
+                    double x[kAhead][4];
 #pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        if (k0 + j < P.K) mx = fmax(mx, fabs(row[koffset(P, mode, koff, k0 + j)]));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-            if (valid && c == 0 && mx > 0.0) {
-                int e;
-                frexp(mx, &e);
-                atomicMax(&tab[gidx[P.g_off + r]], smp ? e + 1 : e);   // one binade of headroom
-            }
+                    for (int q = 0; q < kAhead; q++) load4(row, k0 + q * step, x[q]);
+#pragma unroll
+                    for (int q = 0; q < kAhead; q++)
+#pragma unroll
+                        for (int j = 0; j < 4; j++) m.take(x[q][j]);
+                }
+            m.join(1);
+            m.join(2);
+            m.join(4);
+            if (valid && c == 0 && (m.hi | m.lo) != 0)
+                atomicMax(&tab[gidx[P.g_off + r]], m.exponent() + (smp ? 1 : 0));      // one binade of headroom
             continue;
         }
-        const int nkt = (P.K + 15) >> 4;
-        const int ntile = ((un.z + 7) >> 3) * nkt;
-        for (int t = warp; t < ntile; t += kSplitWarps) {
-            const int rg = t / nkt, kt = t - rg * nkt;
-            const int rl = rg * 8 + lrow, r = un.y + rl;
-            const bool valid = rl < un.z && r < P.rows;
-            double mx = 0.0;
-            if (valid) {
-                const double *row = src + roff[rl];
-                const int k0 = kt * 16 + kq * 4;
+        const int nkt = (K + 15) >> 4, ngroups = (un.z + 7) >> 3;
+        // every kSplitWarps-th core tile, row group by row group; a running
+        // maximum while the warp stays on its rows
+        int rg = 0, kt = warp, cur = -1;
+        RowMax m;
+        auto flush = [&]() {
+            m.join(1);
+            m.join(2);
+            if (kq == 0 && (m.hi | m.lo) != 0) atomicMax(&rexp[cur * 8 + lrow], m.exponent());
+            m = RowMax();
+        };
+        while (kt >= nkt) { kt -= nkt; rg++; }
+        for (; rg < ngroups;) {
+            if (rg != cur) {                                  // uniform over the warp
+                if (cur >= 0) flush();
+                cur = rg;
+            }
+            const int64_t ro = rg * 8 + lrow < un.z ? roff[rg * 8 + lrow] : -1;
+            if (ro >= 0) {
+                double x[4];
+                load4(src + ro, kt * 16 + kq * 4, x);
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (k0 + j < P.K) mx = fmax(mx, fabs(row[koffset(P, mode, koff, k0 + j)]));
+                for (int j = 0; j < 4; j++) m.take(x[j]);
             }
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            if (valid && kq == 0 && mx > 0.0) {
-                int e;
-                frexp(mx, &e);                                 // mx = f * 2^e, f in [0.5, 1)
-                atomicMax(&rexp[rl], e);
-            }
+            kt += kSplitWarps;
+            while (kt >= nkt) { kt -= nkt; rg++; }
         }
+        if (cur >= 0) flush();
         __syncthreads();
         for (int i = threadIdx.x; i < un.z; i += blockDim.x) {
             const int r = un.y + i;
