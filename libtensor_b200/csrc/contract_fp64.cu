@@ -554,6 +554,10 @@ int tile_cfg_bn(int cfg) {
     const int v[] = {Cfg0::BN, Cfg1::BN, Cfg2::BN, Cfg3::BN, Cfg4::BN, Cfg5::BN, Cfg6::BN, Cfg7::BN, Cfg8::BN, Cfg9::BN, Cfg10::BN, Cfg11::BN, Cfg12::BN, Cfg13::BN, Cfg14::BN, Cfg15::BN, Cfg16::BN, Cfg17::BN, Cfg18::BN, Cfg19::BN, Cfg20::BN, Cfg21::BN};
     return v[cfg];
 }
+int tile_cfg_minb(int cfg) {
+    const int v[] = {Cfg0::MINB, Cfg1::MINB, Cfg2::MINB, Cfg3::MINB, Cfg4::MINB, Cfg5::MINB, Cfg6::MINB, Cfg7::MINB, Cfg8::MINB, Cfg9::MINB, Cfg10::MINB, Cfg11::MINB, Cfg12::MINB, Cfg13::MINB, Cfg14::MINB, Cfg15::MINB, Cfg16::MINB, Cfg17::MINB, Cfg18::MINB, Cfg19::MINB, Cfg20::MINB, Cfg21::MINB};
+    return v[cfg];
+}
 
 cudaError_t launch_split_reduce(const DSplit *splits, int32_t nsplits, const DCBlock *cblks,
     const DStack *stacks, const int32_t *stab, const double *ws, int32_t bm, int32_t bn, double *c, int32_t add, cudaStream_t s) {

@@ -29,6 +29,7 @@ namespace ltg {
 int tile_cfg_count();
 int tile_cfg_bm(int cfg);
 int tile_cfg_bn(int cfg);
+int tile_cfg_minb(int cfg);
 }
 
 using namespace ltg;
@@ -522,30 +523,26 @@ int32_t vec16_ok(int64_t off, const SubDims &rows, const SubDims &k, bool second
 // shape with the least padded work, weighted by the relative efficiency of
 // the shape (larger tiles reuse more data per load).  An autotuned table
 // (ltg_autotune) overrides the weights with measured rates.
-struct TileShape { int bm, bn; double eff; };
 constexpr int kNumShapes = 22;
-const TileShape kShapes[kNumShapes] = {
-    {128, 128, 1.00}, {64, 64, 0.78}, {64, 128, 0.90}, {32, 32, 0.45},
-    {80, 128, 0.97}, {96, 128, 0.98}, {48, 128, 0.85}, {112, 128, 0.99},
-    {16, 128, 0.50}, {32, 128, 0.70}, {80, 192, 0.96}, {80, 192, 0.95},
-    {80, 192, 0.94}, {80, 128, 0.93}, {96, 128, 0.92},
-    {80, 128, 0.91}, {80, 192, 0.91}, {64, 128, 1.10},
-    {80, 128, 1.00}, {80, 128, 0.95}, {64, 128, 1.05}, {128, 64, 1.05},
-};
-// relative rates (the m8n8k4 shapes with two CTAs per SM measured fastest:
-// 64 x 128 at 30.1 TFLOP/s on a dense 6144^3 product against 26.1 for the
-// best m16n8k8 shape)
-double g_tile_eff[kNumShapes] = {1.00, 0.78, 0.90, 0.45, 0.97, 0.98, 0.85, 0.99, 0.50, 0.70, 0.96, 0.95,
-                                 0.94, 0.93, 0.92, 0.91, 0.91, 1.10, 1.00, 0.95, 1.05, 1.05};
+// Relative rates of the shapes per padded element.  The m8n8k4 shapes with two
+// CTAs per SM (17-21) from the ladder o=40 v=240 (10.39 ms in shape 18, 10.47 in
+// 19, 10.96 in 20, 11.10 in 17, whose 64-row tiles pad 400 rows to 448), the
+// others from the same runs (11: 11.65, 16: 11.89, 12: 11.95) and from shorter
+// rows (8, 9, 3: blocks of 16, 32 and 25 rows).
+double g_tile_eff[kNumShapes] = {0.80, 0.60, 0.75, 0.35, 0.87, 0.80, 0.70, 0.85, 0.45, 0.60, 0.88, 0.89,
+                                 0.87, 0.87, 0.80, 0.87, 0.87, 1.05, 1.00, 0.99, 1.06, 1.03};
 
-int pick_tile(int64_t M, int64_t N) {
+// (K: contracted length.  Below 256 the start and the epilogue of an item weigh
+// as much as its products, and shape 19's eight warps halve them: o=28 v=220
+// contracted over 110, 142 us against 162 in shape 18 and 172 in 17.)
+int pick_tile(int64_t M, int64_t N, double K) {
     int best = 0;
     double bestc = 1e300;
     for (int c = 0; c < kNumShapes; c++) {
-        const TileShape &s = kShapes[c];
-        double pm = (double)((M + s.bm - 1) / s.bm) * s.bm;
-        double pn = (double)((N + s.bn - 1) / s.bn) * s.bn;
-        double cost = pm * pn / g_tile_eff[c];
+        const int bm = tile_cfg_bm(c), bn = tile_cfg_bn(c);
+        double pm = (double)((M + bm - 1) / bm) * bm;
+        double pn = (double)((N + bn - 1) / bn) * bn;
+        double cost = pm * pn / (c == 19 && K < 256 ? 1.2 * g_tile_eff[c] : g_tile_eff[c]);
         if (cost < bestc) { bestc = cost; best = c; }
     }
     return best;
@@ -651,16 +648,71 @@ void plain_stacks(const std::vector<DTask> &dt, const std::vector<DCBlock> &dc, 
     }
 }
 
-// Work items of one tile shape, appended to `items` costliest first (LPT
-// order for the persistent work queue).  The tail of a launch is uneven when
-// its items are few and long; cutting the k range of the last items into
-// equal chunks (partial tiles summed in chunk order by the split reduction,
-// so results do not depend on scheduling) evens it out at the price of the
-// partial tiles' traffic.  split_k 0 picks, among "no split" and the last
-// 1, 2 or 4 waves' items (or all) in 2-4 chunks, the shortest launch:
-// the slowest SM's work in a simulated greedy assignment (the device's
-// work-queue order) at the nominal per-SM DMMA rate, plus the partial tiles'
-// bytes at HBM speed; 1 never splits; 2-4 split every item in that many.
+// Which of a launch's items (costliest first, costs in padded multiply-adds, nkt
+// k tiles each) have their k range cut, and into how many chunks: those from
+// `first` on into sk.  The tail of a launch is uneven when its items are few and
+// long; chunks (partial tiles summed in chunk order by the split reduction, so
+// results do not depend on scheduling) even it out at the price of the partial
+// tiles' traffic.  split_k 0 picks, among "no split" and the last 1, 2 or 4
+// rounds' items (or all) in 2-4 chunks, the shortest launch: the slowest CTA's
+// work in a simulated greedy assignment (the device's work-queue order) plus the
+// partial tiles' bytes at HBM speed; 1 never splits; 2-4 split every item in
+// that many.  Each resident CTA has its share of an SM's rate whether the others
+// run or not -- a CTA of four warps alone reaches a third of it: 176 items of o=10
+// v=160 in blocks of 5 and 40 take 1182 us whole in shape 18, 784 in four chunks,
+// where one server per SM at the full rate predicts no gain.
+struct SplitChoice {
+    size_t first;
+    int sk;
+    double sec;                       // estimated time of the launch
+};
+SplitChoice choose_split(int cfg, const std::vector<std::pair<double, DItem>> &v, const std::vector<int32_t> &nkt,
+                         int nsm, int split_k) {
+    const size_t n = v.size();
+    const int bm = tile_cfg_bm(cfg), bn = tile_cfg_bn(cfg), minb = tile_cfg_minb(cfg), slots = std::max(1, nsm) * minb;
+    const double rate = 0.8 * 40e12 / 2 / 148 * g_tile_eff[cfg] / minb;      // multiply-adds per second and CTA
+    const double kBytesPerSec = 6e12, kReduceLaunchSec = 4e-6, kItemSec = 2e-6;
+    auto evaluate = [&](size_t first, int sk) {
+        std::vector<double> w;
+        double bytes = 0;
+        for (size_t i = 0; i < n; i++) {
+            const int parts = i >= first ? std::max(1, std::min(sk, nkt[i])) : 1;
+            for (int p = 0; p < parts; p++) w.push_back(v[i].first / parts / rate + kItemSec);
+            if (parts > 1) bytes += (double)(2 * parts + 1) * bm * bn * 8;
+        }
+        std::sort(w.rbegin(), w.rend());
+        std::priority_queue<double, std::vector<double>, std::greater<double>> load;
+        for (int k = 0; k < slots; k++) load.push(0.0);
+        double mk = 0;
+        for (double x : w) {
+            double t = load.top() + x;
+            load.pop();
+            load.push(t);
+            mk = std::max(mk, t);
+        }
+        return mk + (bytes > 0 ? bytes / kBytesPerSec + kReduceLaunchSec : 0.0);
+    };
+    SplitChoice best{n, 1, 0.0};
+    if (n == 0) return best;
+    if (split_k >= 2) {
+        best.first = 0;
+        best.sk = std::min(split_k, 4);
+        best.sec = evaluate(0, best.sk);
+        return best;
+    }
+    best.sec = evaluate(n, 1);
+    if (split_k == 0)
+        for (int rounds : {1, 2, 4, 0})
+            for (int k = 2; k <= 4; k++) {
+                const size_t fs = rounds == 0 ? 0 : (n > (size_t)rounds * slots ? n - (size_t)rounds * slots : 0);
+                const double t = evaluate(fs, k);
+                if (t < best.sec * 0.995) best = {fs, k, t};
+            }
+    return best;
+}
+
+// Work items of one tile shape, appended to `items` costliest first (LPT order
+// for the persistent work queue), some cut into k chunks (choose_split).
 void append_launch(int cfg, std::vector<std::pair<double, DItem>> &v, const std::vector<DTask> &dt,
                    const std::vector<DCBlock> &dc, const PlainStacks &ps, int nsm, int split_k, std::vector<DItem> &items,
                    std::vector<DSplit> &splits, int64_t &ws_elems, std::vector<DmmaLaunch> &launches) {
@@ -675,41 +727,9 @@ void append_launch(int cfg, std::vector<std::pair<double, DItem>> &v, const std:
         const DCBlock &b = dc[ps.first_block(v[i].second.stack)];
         for (int32_t t = b.t_begin; t < b.t_end; t++) nkt[i] += (dt[t].K + bk - 1) / bk;
     }
-    const double kFmaPerSmSec = 40e12 / 2 / 148, kBytesPerSec = 6e12, kReduceLaunchSec = 4e-6;
-    auto evaluate = [&](size_t first_split, int sk) {
-        std::vector<double> w;
-        double bytes = 0;
-        for (size_t i = 0; i < n; i++) {
-            const int parts = i >= first_split ? std::max(1, std::min(sk, nkt[i])) : 1;
-            for (int p = 0; p < parts; p++) w.push_back(v[i].first / parts);
-            if (parts > 1) bytes += (double)(2 * parts + 1) * bm * bn * 8;
-        }
-        std::sort(w.rbegin(), w.rend());
-        std::priority_queue<double, std::vector<double>, std::greater<double>> load;
-        for (int k = 0; k < std::max(1, nsm); k++) load.push(0.0);
-        double mk = 0;
-        for (double x : w) {
-            double t = load.top() + x;
-            load.pop();
-            load.push(t);
-            mk = std::max(mk, t);
-        }
-        return mk / kFmaPerSmSec + (bytes > 0 ? bytes / kBytesPerSec + kReduceLaunchSec : 0.0);
-    };
-    size_t first_split = n;
-    int sk = 1;
-    if (split_k >= 2) {
-        first_split = 0;
-        sk = std::min(split_k, 4);
-    } else if (split_k == 0 && n > 0) {
-        double best = evaluate(n, 1);
-        for (int waves : {1, 2, 4, 0})
-            for (int k = 2; k <= 4; k++) {
-                const size_t fs = waves == 0 ? 0 : (n > (size_t)waves * nsm ? n - (size_t)waves * nsm : 0);
-                const double t = evaluate(fs, k);
-                if (t < best * 0.995) { best = t; first_split = fs; sk = k; }
-            }
-    }
+    const SplitChoice choice = choose_split(cfg, v, nkt, nsm, split_k);
+    const size_t first_split = choice.first;
+    const int sk = choice.sk;
     DmmaLaunch L;
     L.cfg = cfg;
     L.item0 = (int32_t)items.size();
@@ -828,7 +848,7 @@ void stack_items(const ltg_plan *pl, const PlainStacks &ps, const std::vector<CB
     for (size_t k = 0; k < ps.stacks.size(); k++) {
         const DStack &st = ps.stacks[k];
         const CBlockTask &b = cbt[ps.first_block((int32_t)k)];
-        int cfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(st.M, st.N);
+        int cfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(st.M, st.N, b.kflops);
         auto ov = pl->tile_override.find({st.M, st.N});
         if (pl->forced_tile < 0 && ov != pl->tile_override.end()) cfg = ov->second;
         const int bm = tile_cfg_bm(cfg), bn = tile_cfg_bn(cfg);
@@ -1509,7 +1529,7 @@ void build_plain_groups(ltg_plan *pl, const BlockTensorHost &ch, const std::vect
             const double w = (double)lay.rows * lay.cols * lay.kt;
             if (w > best) {
                 best = w;
-                gcfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(lay.rows, lay.cols);
+                gcfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(lay.rows, lay.cols, (double)lay.kt);
                 auto ov = pl->tile_override.find({lay.rows, lay.cols});
                 if (pl->forced_tile < 0 && ov != pl->tile_override.end()) gcfg = ov->second;
             }
@@ -3936,7 +3956,7 @@ int ltg_contract2_autotune(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nsli
         for (auto &o : order) {
             auto key = o.second;
             double best = 1e300;
-            int bestc = pick_tile(key.first, key.second);
+            int bestc = pick_tile(key.first, key.second, 1e9);
             for (int cfg = 0; cfg < tile_cfg_count(); cfg++) {
                 plan->tile_override[key] = cfg;
                 double ms = timed();
