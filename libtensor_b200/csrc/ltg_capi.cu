@@ -1946,7 +1946,7 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
         double most = 0, all = 0;
         for (size_t i = 0; i < n; i += ncta) all += iv[i].first * L;
         if (all <= 1.1 * total / ncta) whole = n;
-        while (whole + ncta <= n && (most += iv[whole].first * L) <= total / ncta) whole += ncta;
+        while (ncta > 0 && whole + ncta <= n && (most += iv[whole].first * L) <= total / ncta) whole += ncta;
         for (size_t i = 0; i < whole; i++) {
             lists[i % ncta].push_back((int32_t)i);
             lists[i % ncta].push_back(L << 8);

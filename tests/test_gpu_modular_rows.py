@@ -49,6 +49,28 @@ def test_redone_rows_take_their_short_panels_along(vir):
     ctx.close()
 
 
+def test_no_products_leave_or_zero_the_result():
+    """An operand without non-zero blocks: the schedule is empty, so adding
+    leaves the result as it is and assigning zeroes it."""
+    ctx = Context(0)
+    cfg = S.LadderConfig("empty", [3], [5, 4])
+    A, B = block_tensor(ctx, cfg.t_spec()), block_tensor(ctx, cfg.v_spec())
+    A.set_zero()
+    B.fill_seeded(23, cfg.v_scale)
+    op = btod_contract2(contraction2(2, 2, 2).contract(2, 2).contract(3, 3), A, B, kc=cfg.kc)
+    C = op.make_result()
+    C.upload(np.full(C.nelems, 3.0))
+    op.perform(C, 1.0, mode=MODE_OZAKI_CRT, nslices=13)
+    ctx.synchronize()
+    assert all(np.all(blk == 3.0) for _, blk in C.blocks(C.download()))
+    op.perform(C, mode=MODE_OZAKI_CRT, nslices=13)
+    ctx.synchronize()
+    assert not any(np.any(blk) for _, blk in C.blocks(C.download())) and C.nonzero() == []
+    for x in (op, C, A, B):
+        x.close()
+    ctx.close()
+
+
 @pytest.mark.parametrize("moduli", range(8, 17))
 @pytest.mark.parametrize("m,n", [(300, 40), (37, 259), (1, 130)], ids=["rows long", "columns long", "one row"])
 def test_recombination_is_exact_on_integers(moduli, m, n):
