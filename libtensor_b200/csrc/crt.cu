@@ -335,17 +335,23 @@ __device__ __forceinline__ uint32_t pack4(uint32_t a, uint32_t b, uint32_t c, ui
 // Sampled rows (sampled_panel): their residues are formed with the sampled
 // bound e (|x| < 2^e unless the sample missed the row's largest elements),
 // and the row's exact exponent goes to the side's second table (ext / eyt).
-// With redo set, only the rows of C whose exact exponent exceeds the bound run
+// With redo, only the rows of C whose exact exponent exceeds the bound run
 // again, in every panel that feeds them (the sampled ones, whose integers may
 // have exceeded 2^P, and the short ones beside them, which must share the
 // row's scaling): with the exact exponent, overwriting the residues formed
-// before.
-template<int L>
+// before.  Most calls redo nothing, and the launch returns at once unless the
+// first pass raised redo_flag; otherwise the few rows concerned are long, so
+// the CTA's threads share each of them (a row's 8 threads alone took 109 us
+// for the rounding noise in otherwise zero amplitude rows of a coupled cluster
+// iteration at o=30 v=300, 45000 words each; 42 us this way).  An instantiation
+// of its own: beside the redo's code the first pass ran 3 % slower.
+template<int L, bool redo>
 __global__ void __launch_bounds__(kSplitThreads, 4)
 crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ units, int32_t nunits,
                const double *__restrict__ A, const double *__restrict__ B, const int32_t *__restrict__ gidx,
                const int32_t *__restrict__ ex, const int32_t *__restrict__ ey, int32_t *ext, int32_t *eyt,
-               int32_t sample, int32_t redo, uint8_t *__restrict__ res, const CrtParams cp) {
+               int32_t *redo_flag, int32_t sample, uint8_t *__restrict__ res, const CrtParams cp) {
+    if (redo && *redo_flag == kNoExp) return;
     __shared__ int32_t koff[kKoffMax];
     __shared__ int64_t roff[kUnitRowsMax];                  // tile mapping: the unit's row offsets
     __shared__ int32_t rexp[kUnitRowsMax];                  //   and exponents
@@ -353,6 +359,20 @@ crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const int4 un = units[u];
         const DCrtPanel &P = panels[un.x];
+        // redo of a row-mapped unit (at most 32 rows): the rows concerned, one
+        // bit each, the same in every warp, and lane i's row's exact exponent
+        uint32_t todo = 0;
+        int e_exact = kNoExp;
+        if (redo && un.w == kUnitRowMap) {
+            bool need = false;
+            if (lane < un.z && un.y + lane < P.rows) {
+                const int g = gidx[P.g_off + un.y + lane];
+                e_exact = (P.side == 0 ? ext : eyt)[g];
+                need = e_exact > (P.side == 0 ? ex : ey)[g];
+            }
+            todo = __ballot_sync(0xffffffffu, need);
+            if (todo == 0) continue;
+        }
         // tabulated k offsets and the tile mapping's row tables (uniform)
         const bool shared = P.nk != 1 || P.kstr[0] != 1 || un.w == kUnitTileMap;
         if (shared) __syncthreads();                         // the previous unit's readers are done
@@ -467,32 +487,29 @@ crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
             // largest |x| of the row as the largest high word without its
             // sign bit (ordered as |x|; its exponent field is that of the maximum)
             uint32_t mx = 0;
-            if (rv) {
-                bool act = true;
-                int e_over = kNoExp;
-                if (redo) {
-                    // the exact exponent against the bound the residues used
-                    const int g = gidx[P.g_off + r];
-                    e_over = tabt[g];
-                    act = e_over > tab[g];
-                }
-                if (act) {
-                    set_row(r, e_over);
-                    const bool track = smp && !redo;
-                    auto run = [&](auto fast_c) {
-                        for (int k0 = 4 * c; k0 < P.wk; k0 += 32) {
-                            double x[4];
-                            load4_if(k0, x, track);
-                            if (track)
+            const bool track = smp && !redo;
+            // words 4 k, 4 (k + step), ... of row q
+            auto run = [&](auto fast_c, int q, int k, int step) {
+                for (int k0 = 4 * k; k0 < P.wk; k0 += 4 * step) {
+                    double x[4];
+                    load4_if(k0, x, track);
+                    if (track)
 #pragma unroll
-                                for (int j = 0; j < 4; j++)
-                                    mx = max(mx, (uint32_t)__double2hiint(x[j]) & 0x7fffffffu);
-                            put4g(fast_c, r, k0, x);
-                        }
-                    };
-                    if (fast) run(std::true_type());
-                    else run(std::false_type());
+                        for (int j = 0; j < 4; j++)
+                            mx = max(mx, (uint32_t)__double2hiint(x[j]) & 0x7fffffffu);
+                    put4g(fast_c, q, k0, x);
                 }
+            };
+            if (redo) {
+                for (uint32_t m = todo; m != 0; m &= m - 1) {
+                    const int i = __ffs(m) - 1;
+                    set_row(un.y + i, __shfl_sync(0xffffffffu, e_exact, i));
+                    run(std::false_type(), un.y + i, threadIdx.x, kSplitThreads);
+                }
+            } else if (rv) {
+                set_row(r, kNoExp);
+                if (fast) run(std::true_type(), r, c, 8);
+                else run(std::false_type(), r, c, 8);
             }
             if (smp && !redo) {
                 // the row's exact exponent (all 8 threads of every row of the warp take part)
@@ -503,7 +520,9 @@ crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
                     // frexp's exponent of a normal number with biased exponent b is
                     // b - 1022; subnormals (b = 0) take -1022, above their own
                     const int b = (int)(mx >> 20);
-                    atomicMax(&tabt[gidx[P.g_off + r]], (b > 0 ? b : 1) - 1022);
+                    const int g = gidx[P.g_off + r], et = (b > 0 ? b : 1) - 1022;
+                    atomicMax(&tabt[g], et);
+                    if (et > tab[g]) *redo_flag = 1;
                 }
             }
             continue;
@@ -1218,12 +1237,17 @@ cudaError_t launch_crt_fused(int shape, const DCrtPanel *panels, const DCrtFamil
 
 cudaError_t launch_crt_residues(const DCrtPanel *panels, const int4 *units, int32_t nunits,
                                 const double *a, const double *b, const int32_t *gidx, const int32_t *ex,
-                                const int32_t *ey, int32_t *ext, int32_t *eyt, int32_t sample, int32_t redo,
-                                uint8_t *res, const CrtParams &cp, cudaStream_t s) {
+                                const int32_t *ey, int32_t *ext, int32_t *eyt, int32_t *redo_flag, int32_t sample,
+                                int32_t redo, uint8_t *res, const CrtParams &cp, cudaStream_t s) {
     if (nunits <= 0) return cudaSuccess;
-    const int grid = nunits;                               // one unit per CTA
+    // one unit per CTA, or for the redo a launch that is cheap to find empty
+    const int grid = redo ? std::min(nunits, 8 * num_sms()) : nunits;
     switch (cp.L) {
-#define CASE_L(n) case n: crt_res_kernel<n><<<grid, kSplitThreads, 0, s>>>(panels, units, nunits, a, b, gidx, ex, ey, ext, eyt, sample, redo, res, cp); break;
+#define CASE_L(n) \
+    case n: \
+        if (redo) crt_res_kernel<n, true><<<grid, kSplitThreads, 0, s>>>(panels, units, nunits, a, b, gidx, ex, ey, ext, eyt, redo_flag, sample, res, cp); \
+        else crt_res_kernel<n, false><<<grid, kSplitThreads, 0, s>>>(panels, units, nunits, a, b, gidx, ex, ey, ext, eyt, redo_flag, sample, res, cp); \
+        break;
     CASE_L(8) CASE_L(9) CASE_L(10) CASE_L(11) CASE_L(12) CASE_L(13) CASE_L(14) CASE_L(15) CASE_L(16)
 #undef CASE_L
     default: return cudaErrorInvalidValue;

@@ -263,7 +263,8 @@ struct CrtExec {
     int32_t *ey() const { return ex() + std::max<int32_t>(nx, 1); }
     int32_t *ext() const { return ey() + std::max<int32_t>(ny, 1); }
     int32_t *eyt() const { return ext() + std::max<int32_t>(nx, 1); }
-    int64_t nexps() const { return 2 * ((int64_t)std::max<int32_t>(nx, 1) + std::max<int32_t>(ny, 1)); }
+    int32_t *redo_flag() const { return eyt() + std::max<int32_t>(ny, 1); }   // set when a sampled bound was too small
+    int64_t nexps() const { return 2 * ((int64_t)std::max<int32_t>(nx, 1) + std::max<int32_t>(ny, 1)) + 1; }
     // row families split in one read (launch_crt_fused): families, their
     // panels and tile offsets, and the 8-row units
     DevBuf fams, famp, famt, funits;
@@ -2799,7 +2800,7 @@ void run_crt(ltg_plan *plan, CrtExec *cx, double *carena, int add, const CrtDest
     for (int redo = 0; redo <= cx->sampled; redo++)
         LTG_CUDA(launch_crt_residues(cx->panels.as<DCrtPanel>(), cx->units.as<int4>(), cx->nunits, pa, pb,
                                      cx->gidx.as<int32_t>(), cx->ex(), cx->ey(),
-                                     cx->ext(), cx->eyt(), cx->sampled, redo,
+                                     cx->ext(), cx->eyt(), cx->redo_flag(), cx->sampled, redo,
                                      cx->res.as<uint8_t>(), cx->cp, s));
     t_split.done();
     TimedLaunch t_gemm(ctx, LTG_KERNEL_OZ_GEMM);

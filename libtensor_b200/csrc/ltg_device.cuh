@@ -378,12 +378,14 @@ cudaError_t launch_crt_fused(int shape, const DCrtPanel *panels, const DCrtFamil
     const int32_t *famt, const int4 *units, int32_t nunits, const double *a, const double *b,
     const int32_t *gidx, int32_t *ex, int32_t *ey, uint8_t *res, const CrtParams &cp, cudaStream_t s);
 // sample != 0: sampled rows also form their exact exponents into ext / eyt
-// (set to "no element" before); redo != 0: only the rows whose exact exponent
-// exceeds their bound run, in every panel, with the exact exponent.
+// (set to "no element" before) and raise redo_flag ("no element" before) where
+// one exceeds its bound; redo != 0: only the rows whose exact exponent exceeds
+// their bound run, in every panel, with the exact exponent, and none if
+// redo_flag was not raised.
 cudaError_t launch_crt_residues(const DCrtPanel *panels, const int4 *units, int32_t nunits,
     const double *a, const double *b, const int32_t *gidx, const int32_t *ex, const int32_t *ey,
-    int32_t *ext, int32_t *eyt, int32_t sample, int32_t redo, uint8_t *res, const CrtParams &cp,
-    cudaStream_t s);
+    int32_t *ext, int32_t *eyt, int32_t *redo_flag, int32_t sample, int32_t redo, uint8_t *res,
+    const CrtParams &cp, cudaStream_t s);
 // Products: ncta persistent CTAs, CTA b working through the pairs
 // (item, first modulus | end modulus << 8) at cta_items[j], j in
 // [cta_items[b], cta_items[b + 1]).

@@ -49,6 +49,41 @@ def test_redone_rows_take_their_short_panels_along(vir):
     ctx.close()
 
 
+def test_redo_follows_the_operands_of_each_call():
+    """One plan, called with operands whose sampled bounds are too small, then
+    with bounds that hold, then too small again: whether rows are redone is
+    found anew in each call, so every result has the bits of a fresh plan's
+    (the integers are exact, nothing depends on timing)."""
+    ctx = Context(0)
+    cfg = S.LadderConfig("redo", [3], [34])
+    A, B = block_tensor(ctx, cfg.t_spec()), block_tensor(ctx, cfg.v_spec())
+    A.fill_seeded(11, cfg.t_scale)
+    plain = B.fill_seeded_host(23, cfg.v_scale)
+    planted = plain.copy()
+    B.upload(plain)
+    for bidx, blk in B.blocks(planted):
+        rows = blk.reshape(blk.shape[0] * blk.shape[1], -1)
+        rows[:, 40] = 8192.0 * float(np.max(np.abs(rows)))
+
+    def plan():
+        op = btod_contract2(contraction2(2, 2, 2).contract(2, 2).contract(3, 3), A, B, kc=cfg.kc)
+        return op, op.make_result()
+
+    kept, C = plan()
+    for arena in (planted, plain, planted, plain):
+        B.upload(arena)
+        fresh, D = plan()
+        for op, r in ((kept, C), (fresh, D)):
+            op.perform(r, mode=MODE_OZAKI_CRT, nslices=13)
+        ctx.synchronize()
+        assert np.array_equal(C.download(), D.download())
+        for x in (fresh, D):
+            x.close()
+    for x in (kept, C, A, B):
+        x.close()
+    ctx.close()
+
+
 def test_no_products_leave_or_zero_the_result():
     """An operand without non-zero blocks: the schedule is empty, so adding
     leaves the result as it is and assigning zeroes it."""
