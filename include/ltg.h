@@ -314,12 +314,13 @@ int ltg_contract2_set_crt_stage(ltg_plan *plan, int32_t kblocks);
  * flops of the blocks they cover.  Needs no device.  Any pointer may be NULL. */
 int ltg_contract2_group_info(ltg_plan *plan, ltg_bt *c, int64_t *ngroups, int64_t *nblocks,
                              double *grouped_flops, double *block_flops);
-/* Autotuner: for every distinct C-block shape (M, N) of the plan, costliest
+/* Autotuner: for every distinct shape (M, N) of the plan's stacks of C blocks (one
+ * block, or blocks that share operand rows and columns task by task), costliest
  * first, times each compiled tile shape on the real contraction (reps calls,
  * CUDA events) and keeps the fastest.  Overwrites c. */
 int ltg_contract2_autotune(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nslices,
                            double ka, double kb, double kc, int32_t reps);
-/* Autotuned table: C-block shape -> tile shape index. */
+/* Autotuned table: stack shape -> tile shape index. */
 int ltg_plan_tiles(ltg_plan *plan, int64_t *m, int64_t *n, int32_t *cfg, int64_t cap,
                    int64_t *count);
 

@@ -576,7 +576,7 @@ struct PlainStacks {
 // distinct A parts and B parts is one stack, else each of its columns is.
 // A ladder's occupied-pair blocks share every V block: ij blocks of 36, 42 and 49
 // rows fill 64-row tiles to 66 %, stacked (127 and 169 rows) to 93 %
-// (o=26 v=130 in blocks of 7, 6 and 29, 23, 13: 917 to 518 us with the cheaper epilogue).
+// (o=26 v=130 in blocks of 7, 6 and 29, 23, 13: 914 to 509 us with the cheaper epilogue).
 void plain_stacks(const std::vector<DTask> &dt, const std::vector<DCBlock> &dc, const std::vector<char> &use,
                   PlainStacks &ps) {
     auto put = [](std::string &k, const void *p, size_t n) { k.append(static_cast<const char *>(p), n); };
@@ -1929,9 +1929,9 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
     // are dealt so, and the other items one modulus at a time, each to the CTA
     // with the least work so far: a contraction with fewer items than SMs would
     // leave most of them idle (ladder o=20 v=90, 43 items: 158 us whole, 46 by
-    // modulus; ring D2h o=46 v=296, 202 uneven items: 195 and 144).  Below 10 % the
-    // sharing is worth more: the ladder o=40 v=240 (566 items, 8 % over) ran
-    // 1.79 ms whole on every GPU, and 1.78 to 2.06 by modulus depending on it.
+    // modulus; ring D2h o=46 v=296, 202 uneven items: 195 and 144).  Below 10 %
+    // the sharing makes up for the uneven end: ladder o=40 v=240 (566 items, 8 %
+    // over) 1.73 ms whole and 1.72 by modulus, o=30 v=300 2.34 and 2.39.
     // cta_items holds the ncta + 1 list offsets (into itself), then the lists'
     // pairs (item, first modulus | end modulus << 8).
     const int32_t ncta = (int32_t)std::min<size_t>(items.size() * L, (size_t)nsm);
