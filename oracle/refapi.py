@@ -50,6 +50,12 @@ _SIGS = {
     "ref_dotprod": (C.c_int, [_vp, _i32p, _vp, _i32p, _dblp]),
 }
 
+
+
+class Missing(FileNotFoundError):
+    """The reference library has not been built (no sources to build it from)."""
+
+
 _lib = None
 DEFAULT_BATCH_SIZE = 1 << 24
 
@@ -61,6 +67,8 @@ def available() -> bool:
 def lib():
     global _lib
     if _lib is None:
+        if not available():
+            raise Missing("oracle/_ref not built")
         # The bundled OpenBLAS finds its libgfortran/libquadmath next to it.
         names = os.listdir(os.path.dirname(LIB_PATH))
         for prefix in ("libquadmath-", "libgfortran-"):
