@@ -244,7 +244,11 @@ int ltg_plan_pairs(ltg_plan *plan, int64_t i, int64_t *out, int64_t cap, int64_t
 int ltg_plan_flops(ltg_plan *plan, double *flops);
 /* perform(): C = kc * contr(ka*A, kb*B) (add == 0), or C += d * ... (add).
  * nslices is the slice count of the split-precision modes (ignored by
- * LTG_MODE_PLAIN_FP64). */
+ * LTG_MODE_PLAIN_FP64).
+ * NaNs and infinities: the plain mode is FP64 arithmetic; the slice modes give
+ * NaN in every element of C whose products read one; the modular mode has no
+ * value for it, and the elements of C that read one are undefined.  In every
+ * mode the other elements of C are as without it. */
 int ltg_contract2(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nslices,
                   double ka, double kb, double kc, int32_t add, double d);
 /* Bytes the split pass(es) of a split-precision mode move for this call:

@@ -74,6 +74,11 @@ __host__ __device__ constexpr bool two_pieces(int sa) { return (S - sa) * oz_max
 constexpr int kMaxStages = 8;
 constexpr int kStageSmem = 200 * 1024;    // shared memory of all stages
 constexpr uint64_t kWaitNs = 2000000000ull;   // 2 s: the drain waits after an abort
+// Rows with a NaN or an infinity: a slice is the low word of an integer and a
+// level sum is joined as integers, so neither can carry one.  The split pass marks
+// the row where its exponent stands, and the products give NaN in what reads it.
+constexpr uint32_t kInfHi = 0x7ff00000u;      // high word of an infinity
+constexpr int32_t kNonFinite = 2000;          // exponent of a marked row (others: -1073 .. 1024)
 
 __device__ __forceinline__ int64_t mixed_offset(int32_t lin, int n, const int32_t *ext,
                                                 const int32_t *str) {
@@ -268,10 +273,12 @@ oz_split_kernel(const DPanel *__restrict__ panels, const int4 *__restrict__ unit
         if (q.rg != cur) {
             cur = q.rg;
             // exponent of the row's largest element (|x| < 2^e): its high word
-            // has it, or, below 2^-1042, the highest low bit of the row
+            // has it, or, below 2^-1042, the highest low bit of the row; a row
+            // with a NaN or an infinity is marked and its slices mean nothing
             int e = 0;
-            if (rhi[i] | rlo[i]) frexp(__hiloint2double((int)rhi[i], (int)rlo[i]), &e);
-            if (r < P.rows && q.kt == 0 && kq == 0) exps[P.exp_off + r] = e;
+            const bool finite = rhi[i] < kInfHi;
+            if (finite && (rhi[i] | rlo[i])) frexp(__hiloint2double((int)rhi[i], (int)rlo[i]), &e);
+            if (r < P.rows && q.kt == 0 && kq == 0) exps[P.exp_off + r] = finite ? e : kNonFinite;
             // 2^(beta0 - e), as two finite factors where one would not do
             const int sh = kBeta0 - e;
             one = sh >= -1000 && sh <= 1000;
@@ -639,7 +646,9 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
                 const DPanel &px = panels[t.px];
                 const DPanel &py = panels[t.py];
                 const int nkb = px.K_pad / kbe;
-                const double f = ldexp(t.coeff, exps[px.exp_off + x] - 2 * beta0);
+                const double nan = __longlong_as_double(0x7ff8000000000000ll);
+                const int ex = exps[px.exp_off + x];
+                const double f = ex == kNonFinite ? nan : ldexp(t.coeff, ex - 2 * beta0);
                 // the columns' exponents, one or two per lane
                 const int32_t *ey = exps + py.exp_off + item.y0 + c0;
                 const int e_lo = lane < hc ? ey[lane] : 0, e_hi = kHalf > 32 && lane + 32 < hc ? ey[lane + 32] : 0;
@@ -665,6 +674,13 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acce_bar);
+                }
+                if (ok && __any_sync(0xffffffffu, e_lo == kNonFinite || e_hi == kNonFinite)) {
+#pragma unroll
+                    for (int j = 0; j < kHalf; j++) {
+                        const int e = __shfl_sync(0xffffffffu, j < 32 ? e_lo : e_hi, j & 31);
+                        if (e == kNonFinite) acc[j] = nan;
+                    }
                 }
             }
             if (!ok) break;
