@@ -60,6 +60,7 @@ constexpr double kMagicD = 6755399441055744.0;      // 1.5 * 2^52: round-to-inte
 constexpr float kMagicF = 12582912.0f;              // 1.5 * 2^23
 constexpr int32_t kNoExp = -1000000;                // exponent of a row with no non-zero element
 constexpr int32_t kKeepRow = -2000000;              // redo pass: a row whose residues stand
+constexpr int32_t kRereadRow = 1000000;             // exponent pass: a row with a NaN or an infinity
 
 // The moduli (pairwise coprime, <= 256) and the constants derived from them,
 // as compile-time functions so that unrolled loops over the moduli fold them
@@ -189,12 +190,22 @@ __device__ __forceinline__ int64_t koffset(const DCrtPanel &P, int mode, const i
 // per thread held the pass to a quarter of the HBM rate (ladder o=20 v=90: 48 us
 // for 78 MB, 20 this way with two 32-byte groups in flight; more of them cost the
 // core tiles of short rows their occupancy; ring D2h 71 to 68 us).
+// NaNs and infinities take no part: integers cannot carry them, so what reads
+// one means nothing, but the row's other elements keep their scale.  A row
+// whose maximum comes out non-finite is read again without them, so that the
+// pass has no test per element.
+constexpr uint32_t kInfHi = 0x7ff00000u;                // high word of an infinity
+__device__ __forceinline__ uint32_t magnitude_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
 struct RowMax {
     uint32_t hi = 0, lo = 0;
     __device__ __forceinline__ void take(double x) {
-        hi = max(hi, (uint32_t)__double2hiint(x) & 0x7fffffffu);
+        hi = max(hi, magnitude_hi(x));
         lo |= (uint32_t)__double2loint(x);
     }
+    __device__ __forceinline__ void take_finite(double x) {
+        if (magnitude_hi(x) < kInfHi) take(x);
+    }
+    __device__ __forceinline__ bool finite() const { return hi < kInfHi; }
     __device__ __forceinline__ void join(int lanes) {
         hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, lanes));
         lo |= __shfl_xor_sync(0xffffffffu, lo, lanes);
@@ -269,6 +280,17 @@ crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
             m.join(1);
             m.join(2);
             m.join(4);
+            if (__any_sync(0xffffffffu, !m.finite())) {
+                RowMax f;
+                if (valid)
+#pragma unroll 1
+                    for (int k0 = 4 * c; k0 < K; k0 += step)
+                        for (int j = 0; j < 4 && k0 + j < K; j++) f.take_finite(row[koffset(P, mode, koff, k0 + j)]);
+                f.join(1);
+                f.join(2);
+                f.join(4);
+                if (!m.finite()) m = f;
+            }
             if (valid && c == 0 && (m.hi | m.lo) != 0)
                 atomicMax(&tab[gidx[P.g_off + r]], m.exponent() + (smp ? 1 : 0));      // one binade of headroom
             continue;
@@ -281,7 +303,8 @@ crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
         auto flush = [&]() {
             m.join(1);
             m.join(2);
-            if (kq == 0 && (m.hi | m.lo) != 0) atomicMax(&rexp[cur * 8 + lrow], m.exponent());
+            if (kq == 0 && (m.hi | m.lo) != 0)
+                atomicMax(&rexp[cur * 8 + lrow], m.finite() ? m.exponent() : kRereadRow);
             m = RowMax();
         };
         while (kt >= nkt) { kt -= nkt; rg++; }
@@ -304,7 +327,15 @@ crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
         __syncthreads();
         for (int i = threadIdx.x; i < un.z; i += blockDim.x) {
             const int r = un.y + i;
-            if (r < P.rows && rexp[i] > kNoExp) atomicMax(&tab[gidx[P.g_off + r]], rexp[i]);
+            if (r >= P.rows || rexp[i] == kNoExp) continue;
+            int e = rexp[i];
+            if (e == kRereadRow) {
+                RowMax f;
+#pragma unroll 1
+                for (int k = 0; k < K; k++) f.take_finite(src[roff[i] + koffset(P, mode, koff, k)]);
+                e = f.exponent();
+            }
+            if (e > kNoExp) atomicMax(&tab[gidx[P.g_off + r]], e);
         }
     }
 }
@@ -496,7 +527,7 @@ crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
                     if (track)
 #pragma unroll
                         for (int j = 0; j < 4; j++)
-                            mx = max(mx, (uint32_t)__double2hiint(x[j]) & 0x7fffffffu);
+                            mx = max(mx, magnitude_hi(x[j]));
                     put4g(fast_c, q, k0, x);
                 }
             };
@@ -516,7 +547,9 @@ crt_res_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
                 mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
                 mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
                 mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-                if (rv && c == 0 && mx != 0) {
+                // (a row with a NaN or an infinity keeps its bound unchecked: what
+                // its other elements would change reads that one too)
+                if (rv && c == 0 && mx != 0 && mx < kInfHi) {
                     // frexp's exponent of a normal number with biased exponent b is
                     // b - 1022; subnormals (b = 0) take -1022, above their own
                     const int b = (int)(mx >> 20);
@@ -596,7 +629,10 @@ crt_fused_kernel(const DCrtPanel *__restrict__ panels, const DCrtFamily *__restr
                     const int k0 = t * FC::kTileK + kq * 4;
 #pragma unroll
                     for (int j = 0; j < 4; j++)
-                        if (k0 + j < P.K) mx = fmax(mx, fabs(row[k0 + j]));
+                        if (k0 + j < P.K) {
+                            const double v = fabs(row[k0 + j]);
+                            mx = fmax(mx, v < HUGE_VAL ? v : 0.0);       // finite elements only, as RowMax
+                        }
                 }
             }
         }

@@ -1,9 +1,10 @@
-"""A NaN or an infinity in an operand: the slice modes give NaN in every element
-of C that reads it, as FP64 arithmetic does, and change no other."""
+"""A NaN or an infinity in an operand, split-precision modes: the slice modes
+give NaN in every element of C that reads it, as FP64 arithmetic does, and no
+mode lets it change an element that does not read it."""
 import numpy as np
 import pytest
 
-from libtensor_b200.core import (MODE_OZAKI_BF16, MODE_OZAKI_FP8, MODE_OZAKI_INT8, Context,
+from libtensor_b200.core import (MODE_OZAKI_BF16, MODE_OZAKI_CRT, MODE_OZAKI_FP8, MODE_OZAKI_INT8, Context,
                                  block_tensor, btod_contract2, contraction2)
 from libtensor_b200.spec import BTSpec
 
@@ -79,4 +80,28 @@ def test_slice_modes_give_nan_where_it_is_read(mode, slices, m, n):
                 reads[:, r] = True
             assert np.all(np.isnan(got[reads])), (bad, side)
             assert np.array_equal(got[~reads], clean[~reads]), (bad, side)
+    ctx.close()
+
+
+@pytest.mark.parametrize("ks,k", [([40, 33], 50), ([40, 1100], 41), ([40, 1100], 40 + 700)],
+                         ids=["exact maxima", "sampled, seen", "sampled, not seen"])
+def test_modular_mode_keeps_the_scale_of_the_finite_elements(ks, k):
+    """Rows of up to 1023 elements have exact maxima, longer ones a bound from
+    elements 0-31, 512-543 and so on, checked by the residue pass.  The result
+    with a zero in the place of the bad element has the same row maxima, so
+    what does not read it has the same bits."""
+    ctx = Context(0)
+    m, n = [130, 5], [20, 3]
+    a, b = _operands(m, n, ks, 5)
+    for bad in BAD:
+        r = m[0] - 1
+        got, clean = _results(ctx, a, b, m, n, ks, bad, 0, (r, k), MODE_OZAKI_CRT, 13)
+        reads = np.zeros(got.shape, bool)
+        reads[r, :n[0]] = True
+        assert np.array_equal(got[~reads], clean[~reads]), bad
+        # products with exact zeros: what is left of the row is finite and right
+        b0 = b.copy()
+        b0[:, k] = 0.0
+        got, clean = _results(ctx, a, b0, m, n, ks, bad, 0, (r, k), MODE_OZAKI_CRT, 13)
+        assert np.array_equal(got, clean), bad
     ctx.close()
