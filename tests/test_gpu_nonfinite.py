@@ -83,18 +83,21 @@ def test_slice_modes_give_nan_where_it_is_read(mode, slices, m, n):
     ctx.close()
 
 
-@pytest.mark.parametrize("ks,k", [([40, 33], 50), ([40, 1100], 41), ([40, 1100], 40 + 700)],
-                         ids=["exact maxima", "sampled, seen", "sampled, not seen"])
-def test_modular_mode_keeps_the_scale_of_the_finite_elements(ks, k):
+@pytest.mark.parametrize("ks,k,big", [([40, 33], 50, 1024.0), ([40, 600], 50, 1024.0), ([40, 1100], 41, 1024.0),
+                                      ([40, 1100], 40 + 700, 1.0)],
+                         ids=["exact, core tiles", "exact, rows", "sampled, seen", "sampled, not seen"])
+def test_modular_mode_keeps_the_scale_of_the_finite_elements(ks, k, big):
     """Rows of up to 1023 elements have exact maxima, longer ones a bound from
     elements 0-31, 512-543 and so on, checked by the residue pass.  The result
-    with a zero in the place of the bad element has the same row maxima, so
-    what does not read it has the same bits."""
+    with a zero in the place of the bad element has the same row maxima (the
+    element beside the bad one, where it is read with it), so what does not read
+    it has the same bits."""
     ctx = Context(0)
     m, n = [130, 5], [20, 3]
     a, b = _operands(m, n, ks, 5)
+    r = m[0] - 1
+    a[r, k ^ 1] = big * np.abs(a[r]).max()
     for bad in BAD:
-        r = m[0] - 1
         got, clean = _results(ctx, a, b, m, n, ks, bad, 0, (r, k), MODE_OZAKI_CRT, 13)
         reads = np.zeros(got.shape, bool)
         reads[r, :n[0]] = True
