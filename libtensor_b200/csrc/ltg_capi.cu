@@ -140,19 +140,24 @@ struct ltg_ctx {
     DevBuf dot_out;              // device scalar for synchronous dot products
     // Workspace of the k-split partial tiles, one for all plans: every launch that
     // fills it and the reduction that reads it follow each other on the context's
-    // stream.  It only grows, at least twofold; outgrown buffers stay until the
-    // context goes (plans and captured graphs point into them), so that all of
-    // them together are at most twice the largest.
-    std::vector<std::unique_ptr<DevBuf>> split_ws;
-    double *split_workspace(int64_t elems) {
+    // stream.  The plans own it: one that a larger need has replaced, or that no
+    // plan uses, is freed with the last plan that points into it (a captured
+    // graph needs its plan in any case).  Only kKeptWs bytes stay with the context,
+    // so that small contractions prepared one after the other do not allocate.
+    static constexpr size_t kKeptWs = (size_t)32 << 20;
+    std::shared_ptr<DevBuf> kept_ws;
+    std::weak_ptr<DevBuf> split_ws;
+    std::shared_ptr<DevBuf> split_workspace(int64_t elems) {
         const size_t need = (size_t)std::max<int64_t>(elems, 0) * sizeof(double);
         if (need == 0) return nullptr;
-        if (split_ws.empty() || split_ws.back()->bytes < need) {
-            std::unique_ptr<DevBuf> b(new DevBuf());
-            b->alloc(std::max(need, split_ws.empty() ? (size_t)4 << 20 : 2 * split_ws.back()->bytes));
-            split_ws.push_back(std::move(b));
+        std::shared_ptr<DevBuf> b = need <= kKeptWs ? kept_ws : split_ws.lock();
+        if (!b || b->bytes < need) {
+            b = std::make_shared<DevBuf>();
+            b->alloc(std::max(need, kKeptWs));
+            if (need <= kKeptWs) kept_ws = b;
+            else split_ws = b;
         }
-        return split_ws.back()->as<double>();
+        return b;
     }
     KernelTiming timing;
     // Bounded device waits of the tcgen05 kernels: the limit of one pipeline
@@ -197,14 +202,16 @@ struct PlainGroups {
     double scale = 1.0;                       // ka kb kc (and d in add mode)
     DevBuf buf, pieces, units, sunits, comps, res_off, ctab, cells;
     DevBuf tasks, cblks, stacks, stab, items, splits;   // DMMA work over buf
-    double *ws = nullptr;                     // in the context's split workspace
+    std::shared_ptr<DevBuf> ws;               // the context's split workspace (null without k chunks)
+    double *ws_at(int64_t off) const { return ws ? ws->as<double>() + off : nullptr; }
     std::vector<DmmaLaunch> launches;
 };
 
 struct ContractExec {
     // device task arrays bound to one output tensor and coefficient set
     DevBuf pack;
-    double *ws = nullptr;                     // in the context's split workspace
+    std::shared_ptr<DevBuf> ws;               // the context's split workspace (null without k chunks)
+    double *ws_at(int64_t off) const { return ws ? ws->as<double>() + off : nullptr; }
     DevPart tasks, cblks, stacks, stab, items, splits;
     std::unique_ptr<PlainGroups> groups;      // grouped small blocks, if any
     std::vector<DmmaLaunch> launches;
@@ -3159,11 +3166,11 @@ int ltg_contract2_symmetrized(ltg_plan *plan, ltg_bt *r, int32_t mode, int32_t n
                                               pg->items.as<DItem>() + l.item0, l.nitems,
                                               ctx->scratch_counter.as<int32_t>() + (slot++ % 64),
                                               pg->buf.as<double>(), pg->buf.as<double>(), pg->buf.as<double>(),
-                                              pg->ws + l.ws_off, 0, l.cfg, s));
+                                              pg->ws_at(l.ws_off), 0, l.cfg, s));
                 if (l.nsplits > 0) {
                     LTG_CUDA(launch_split_reduce(pg->splits.as<DSplit>() + l.split0, l.nsplits, pg->cblks.as<DCBlock>(),
                                                  pg->stacks.as<DStack>(), pg->stab.as<int32_t>(),
-                                                 pg->ws + l.ws_off, tile_cfg_bm(l.cfg),
+                                                 pg->ws_at(l.ws_off), tile_cfg_bm(l.cfg),
                                                  tile_cfg_bn(l.cfg), pg->buf.as<double>(), 0, s));
                     ctx->launches++;
                 }
@@ -3719,11 +3726,11 @@ int ltg_contract2(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nslices, doub
                                               pg->items.as<DItem>() + l.item0, l.nitems,
                                               ctx->scratch_counter.as<int32_t>() + (slot++ % 64),
                                               pg->buf.as<double>(), pg->buf.as<double>(), pg->buf.as<double>(),
-                                              pg->ws + l.ws_off, 0, l.cfg, s));
+                                              pg->ws_at(l.ws_off), 0, l.cfg, s));
                 if (l.nsplits > 0) {
                     LTG_CUDA(launch_split_reduce(pg->splits.as<DSplit>() + l.split0, l.nsplits, pg->cblks.as<DCBlock>(),
                                                  pg->stacks.as<DStack>(), pg->stab.as<int32_t>(),
-                                                 pg->ws + l.ws_off, tile_cfg_bm(l.cfg),
+                                                 pg->ws_at(l.ws_off), tile_cfg_bm(l.cfg),
                                                  tile_cfg_bn(l.cfg), pg->buf.as<double>(), 0, s));
                     ctx->launches++;
                 }
@@ -3737,11 +3744,11 @@ int ltg_contract2(ltg_plan *plan, ltg_bt *c, int32_t mode, int32_t nslices, doub
                                           ex->items.as<DItem>() + l.item0, l.nitems,
                                           ctx->scratch_counter.as<int32_t>() + (slot++ % 64),
                                           plan->a->arena.as<double>(), plan->b->arena.as<double>(),
-                                          c->arena.as<double>(), ex->ws + l.ws_off, add, l.cfg, s));
+                                          c->arena.as<double>(), ex->ws_at(l.ws_off), add, l.cfg, s));
             if (l.nsplits > 0) {
                 LTG_CUDA(launch_split_reduce(ex->splits.as<DSplit>() + l.split0, l.nsplits, ex->cblks.as<DCBlock>(),
                                                  ex->stacks.as<DStack>(), ex->stab.as<int32_t>(),
-                                             ex->ws + l.ws_off, tile_cfg_bm(l.cfg), tile_cfg_bn(l.cfg),
+                                             ex->ws_at(l.ws_off), tile_cfg_bm(l.cfg), tile_cfg_bn(l.cfg),
                                              c->arena.as<double>(), add, s));
                 ctx->launches++;
             }
