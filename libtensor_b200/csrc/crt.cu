@@ -173,9 +173,10 @@ __global__ void crt_fill_kernel(int32_t *p, int32_t n, int32_t v) {
 }
 
 
-// k offset mode of a panel: 0 contiguous, 1 tabulated in koff, 2 computed.
+// k offset mode of a panel: 0 contiguous, 1 tabulated in koff, 2 computed (in 64
+// bits).
 __device__ __forceinline__ int koff_setup(const DCrtPanel &P, int32_t *koff) {
-    const int mode = (P.nk == 1 && P.kstr[0] == 1) ? 0 : (P.K <= kKoffMax ? 1 : 2);
+    const int mode = (P.nk == 1 && P.kstr[0] == 1) ? 0 : (P.K <= kKoffMax && !P.wide ? 1 : 2);
     if (mode == 1)
         for (int k = threadIdx.x; k < P.K; k += blockDim.x) koff[k] = (int32_t)mixed_offset(k, P.nk, P.kext, P.kstr);
     return mode;

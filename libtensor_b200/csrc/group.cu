@@ -47,7 +47,7 @@ gather_cells_kernel(const DGather *__restrict__ pieces, const int4 *__restrict__
         __syncthreads();                                          // the previous unit's readers are done
         if (tab)
             for (int k = threadIdx.x; k < P.K; k += blockDim.x) koff[k] = (int32_t)gmixed(k, P.nk, P.kext, P.kstr);
-        // (offsets inside a block fit 32 bits)
+        // (offsets fit 32 bits: the host groups blocks below 2^31 elements only)
         for (int r = threadIdx.x; r < un.z; r += blockDim.x) roff[r] = (int32_t)gmixed(un.y + r, P.nr, P.rext, P.rstr);
         __syncthreads();
         const double *src = (P.src ? B : A) + P.src_off;

@@ -796,13 +796,6 @@ std::vector<std::pair<int64_t, int64_t>> plain_group_shapes(ltg_plan *pl, ltg_bt
                                                            const std::vector<CBlockTask> &cbt,
                                                            std::vector<int32_t> &group_of);
 
-// Largest offset a sub-dimension group can add (strides s0, or s1).
-int64_t sub_span(const SubDims &s, bool second) {
-    int64_t m = 0;
-    for (int i = 0; i < s.n; i++) m += (int64_t)(s.ext[i] - 1) * (second ? s.s1[i] : s.s0[i]);
-    return m;
-}
-
 // Device task and C-block arrays of the plain path (post: d in add mode,
 // else 1); every address a task can form must lie inside its arena (c_elems:
 // the C arena's size).
@@ -810,9 +803,9 @@ void plain_task_arrays(const ltg_plan *pl, int64_t c_elems, const std::vector<Ge
                        const std::vector<CBlockTask> &cbt, double post, std::vector<DTask> &dt,
                        std::vector<DCBlock> &dc) {
     for (const GemmTask &t : tasks) {
-        int64_t amax = t.a_off + sub_span(t.m, false) + sub_span(t.k, false);
-        int64_t bmax = t.b_off + sub_span(t.n, false) + sub_span(t.k, true);
-        int64_t cmax = t.c_off + sub_span(t.m, true) + sub_span(t.n, true);
+        int64_t amax = t.a_off + t.m.span(false) + t.k.span(false);
+        int64_t bmax = t.b_off + t.n.span(false) + t.k.span(true);
+        int64_t cmax = t.c_off + t.m.span(true) + t.n.span(true);
         if (t.a_off < 0 || amax >= pl->a->h.total_elems || t.b_off < 0 || bmax >= pl->b->h.total_elems ||
             t.c_off < 0 || cmax >= c_elems)
             throw error(kErrState, "contraction task addresses outside an operand arena");
@@ -922,7 +915,7 @@ ContractExec *prepare_exec(ltg_plan *pl, ltg_bt *c, double ka, double kb, double
             auto f = slot_of_off.find(b.c_off);
             if (f == slot_of_off.end()) throw error(kErrBadArg, "a task's c_off is not the start of a block of C");
             if (in_sched[f->second]) throw error(kErrBadArg, "the tasks of one C block must be consecutive");
-            if (b.c_off + sub_span(b.cm, true) + sub_span(b.cn, true) >= b.c_off + c->h.blk_size[f->second] ||
+            if (b.c_off + b.cm.span(true) + b.cn.span(true) >= b.c_off + c->h.blk_size[f->second] ||
                 b.M * b.N > c->h.blk_size[f->second])
                 throw error(kErrBadArg, "a task's C range leaves its block");
             ex->sched_slots.push_back(f->second);
@@ -1004,6 +997,7 @@ OzExec *prepare_ozaki(ltg_plan *pl, ltg_bt *c, int mode, int S, double ka, doubl
         SubDims kk = k;
         if (kb_second) for (int i = 0; i < kk.n; i++) kk.s0[i] = kk.s1[i];
         pack_sub(kk, p.nk, p.kext, p.kstr, nullptr);
+        p.wide = kk.fits_i32(false) ? 0 : 1;
         p.slice_off = slice_bytes;
         slice_bytes += ((int64_t)S * p.rows_pad * p.K_pad * esz + 1023) / 1024 * 1024;
         p.exp_off = exp_rows;
@@ -1437,7 +1431,9 @@ DCrtComp crt_group_tables(const ltg_plan *pl, const BlockTensorHost &ch, const C
 }
 
 // Dense layout of one group for the plain path (element offsets in buf, all
-// multiples of 4): A panel rows x kt, B panel cols x kt, result rows x cols.
+// multiples of 4): A panel rows x kt, B panel cols x kt, result rows x cols, each
+// below 2^31 elements -- so is every block of the group then, and the gather
+// keeps offsets inside a block in 32 bits.
 struct PlainGroupLayout {
     int64_t rows = 0, cols = 0, kt = 0, aoff = 0, boff = 0, coff = 0;
     std::vector<int64_t> rofs, sofs, kofs;
@@ -1707,6 +1703,7 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
         SubDims kk = k;
         if (kb_second) for (int i = 0; i < kk.n; i++) kk.s0[i] = kk.s1[i];
         pack_sub(kk, p.nk, p.kext, p.kstr, nullptr);
+        p.wide = kk.fits_i32(false) ? 0 : 1;
         p.res_off = res_bytes;
         res_bytes += ((int64_t)L * p.rows_pad * p.K_pad + 1023) / 1024 * 1024;
         // the padding rows and k of the image stay zero from the buffer's clearing
@@ -1846,6 +1843,7 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
             q.g_off = rec.g_off + r0;
             pack_sub(cl.rows, q.nr, q.rext, q.rstr, nullptr);
             pack_sub(cl.k, q.nk, q.kext, q.kstr, nullptr);
+            q.wide = cl.k.fits_i32(false) ? 0 : 1;
             if (cl.rows.total() != nrow || cl.k.total() != G.kn[k]) throw error(kErrState, "grouped cell extents");
             q.r0 = r0; q.k0 = kofs[k]; q.wrows = q.rows; q.wk = round4(q.K);
             max_rows = std::max(max_rows, q.wrows);

@@ -94,7 +94,8 @@ struct DPanel {
     int32_t src;                  // 0: A arena, 1: B arena
     int32_t rows, K, rows_pad, K_pad;
     int32_t tr;                   // rows per tile image (128 on the MMA M side, else the N tile width)
-    int32_t nr, nk, pad;
+    int32_t wide;                 // some k offset is beyond 32 bits: they are not tabulated
+    int32_t nr, nk;
     int32_t rext[kDevMaxSub], rstr[kDevMaxSub];
     int32_t kext[kDevMaxSub], kstr[kDevMaxSub];
 };
@@ -130,6 +131,7 @@ struct DCrtPanel {
     int32_t tr;                   // rows per tile image (128, or the N tile width)
     int32_t coef;                 // integer coefficient folded into the residues
     int32_t g_off;                // first of this panel's rows in the global row-index array
+    int32_t wide;                 // some k offset is beyond 32 bits: they are not tabulated
     int32_t nr, nk;
     int32_t rext[kDevMaxSub], rstr[kDevMaxSub];
     int32_t kext[kDevMaxSub], kstr[kDevMaxSub];

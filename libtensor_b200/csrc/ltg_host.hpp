@@ -263,6 +263,16 @@ struct SubDims {
     int64_t s0[kMaxSub] = {};   // stride in the first tensor of the pair
     int64_t s1[kMaxSub] = {};   // stride in the second tensor of the pair
     int64_t total() const { int64_t r = 1; for (int i = 0; i < n; i++) r *= ext[i]; return r; }
+    // Largest offset the group adds in the first (or the second) tensor.
+    int64_t span(bool second) const {
+        int64_t r = 0;
+        for (int i = 0; i < n; i++) r += (int64_t)(ext[i] - 1) * (second ? s1[i] : s0[i]);
+        return r;
+    }
+    // Whether kernels may keep these offsets in 32 bits.  The strides alone do not
+    // tell: contracted over the outermost of a block's dimensions, 100 steps of
+    // 3e7 elements reach beyond 2^31 (a block of 24 GB).
+    bool fits_i32(bool second) const { return span(second) <= INT32_MAX; }
 };
 
 // One GEMM-shaped product of a (C block, coalesced pair):

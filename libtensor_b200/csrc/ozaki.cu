@@ -171,8 +171,8 @@ oz_split_kernel(const DPanel *__restrict__ panels, const int4 *__restrict__ unit
     const int4 un = units[blockIdx.x];
     const DPanel &P = panels[un.x];
     const double *src = (P.src ? B : A) + P.src_off;
-    // k offsets: contiguous, tabulated, or computed per element
-    const int K = P.K, mode = P.nk == 0 || (P.nk == 1 && P.kstr[0] == 1) ? 0 : (K <= kKoffMax ? 1 : 2);
+    // k offsets: contiguous, tabulated, or computed per element (in 64 bits)
+    const int K = P.K, mode = P.nk == 0 || (P.nk == 1 && P.kstr[0] == 1) ? 0 : (K <= kKoffMax && !P.wide ? 1 : 2);
     if (mode == 1)
         for (int k = threadIdx.x; k < K; k += kSplitThreads) koff[k] = (int32_t)mixed_offset(k, P.nk, P.kext, P.kstr);
     for (int i = threadIdx.x; i < un.z; i += kSplitThreads) {
