@@ -57,7 +57,6 @@ constexpr int kEpiWarps = 16;
 constexpr int kGemmThreads = 32 * (kEpiWarps + 2);  // + bulk-copy producer + MMA issuer
 constexpr uint64_t kWaitNs = 2000000000ull;         // 2 s: the drain waits after an abort
 constexpr double kMagicD = 6755399441055744.0;      // 1.5 * 2^52: round-to-integer constant
-constexpr float kMagicF = 12582912.0f;              // 1.5 * 2^23
 constexpr int32_t kNoExp = -1000000;                // exponent of a row with no non-zero element
 constexpr int32_t kKeepRow = -2000000;              // redo pass: a row whose residues stand
 constexpr int32_t kRereadRow = 1000000;             // exponent pass: a row with a NaN or an infinity
@@ -1004,14 +1003,14 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(smem_u32(smem)), "l"(gmem) : "memory");
 }
 
-// The integer X in (-M/2, M/2) with the residues byte(i) mod m_i, rounded to
-// FP64.  The limb sums S_n are exact, q = rint(sum_i r_i W_i / M) is found from
-// the two highest (the host keeps |X| at least 1e-9 M / 2 inside the range, far
-// more than their error), each S_n - q M_n is exact again (q < 2^12), and the
-// limbs join from the top, where only the result is rounded.
-// Bound by FP64 issue: about 60 operations at 13 moduli.  Garner's mixed-radix
-// digits in FP32 took 346 instructions per element of the ring and were issue
-// bound (170 us; 134 us this way; ladder o=40 v=240: 226 to 161 us).
+// The integer X in (-M/2, M/2) with the residues byte(i) mod m_i, in FP64.  The
+// limb sums S_n are exact, q = rint(sum_i r_i W_i / M) is found from the highest
+// limbs, each S_n - q M_n is exact again (q < 2^12), and the limbs join from the
+// top: exact below 2^53, else one rounding per limb joined (one or two, three at
+// 16 moduli).  The host keeps |X| 3.4e-10 M inside the range (1e-9 in log2, and
+// far more at 16 moduli, whose 2^17 products of 50-bit integers end at 2^-7 of
+// M/2).  Two limbs find q to 2e-12, except where the top one has 8 bits or fewer:
+// at 11 moduli what they leave out is 4e-11, so a third is taken there.
 template<int L, class F>
 __device__ __forceinline__ double crt_reconstruct(F &&byte) {
     constexpr int NL = crt_limbs(L);
@@ -1027,8 +1026,12 @@ __device__ __forceinline__ double crt_reconstruct(F &&byte) {
             S[n] = i == 0 ? r * w : fma(r, w, S[n]);
         });
     });
-    constexpr double c1 = crt_limb_share(L, NL - 1), c0 = NL > 1 ? crt_limb_share(L, NL - 2) : 0.0;
-    const double q = fma(S[NL - 1], c1, NL > 1 ? S[NL > 1 ? NL - 2 : 0] * c0 : 0.0) + kMagicD - kMagicD;
+    static_assert(NL >= 2, "8 moduli or more");
+    constexpr bool kThird = NL > 2 && (crt_product(L) >> (kLimbBits * (NL - 1) + 8)) == 0;
+    constexpr double c1 = crt_limb_share(L, NL - 1), c0 = crt_limb_share(L, NL - 2);
+    double low = S[NL - 2] * c0;
+    if constexpr (kThird) low = fma(S[NL - 3], crt_limb_share(L, NL - 3), low);
+    const double q = fma(S[NL - 1], c1, low) + kMagicD - kMagicD;
     double X = 0.0;
     StaticFor<0, NL>::run([&](auto nn) {
         constexpr int n = NL - 1 - decltype(nn)::value;

@@ -1752,7 +1752,7 @@ CrtExec *prepare_crt(ltg_plan *pl, ltg_bt *c, int L, double ka, double kb, doubl
     // |c * x * 2^(P - e)| < 2^50 keeps every residue computation exact (the
     // FP64 round-to-integer trick needs magnitudes below 2^51)
     const int pcap = 50 - (int)std::ceil(std::log2((double)max_coef));
-    // (1e-9 inside the range: the recombination finds X / M in FP64)
+    // (1e-9 bits inside the range, 3.4e-10 M: the recombination finds X / M in FP64)
     const int P = std::min(pcap, (int)std::floor((log2M - 1.0 - 1e-9 - std::log2((double)max_sum)) / 2.0));
     if (P < 24) throw error(kErrUnsupported, "too few moduli for this contraction");
 
