@@ -2142,12 +2142,12 @@ void validate_transfer(const TransferPlan &plan, const std::vector<int64_t> &src
 // coefficients, destination, mode) builds and uploads the task arrays; later
 // calls, including calls inside a CUDA-graph capture, only launch.
 // Device form of a transfer plan: every job seen as planes of A rows x B
-// columns (DJob).  Jobs whose terms all read the columns with unit stride run
-// in row mode (warp items of about kItemElems elements: row chunks x column
-// segments); a job
-// with a transposing term runs in tiled mode, tiles of at most 64x64 whose
-// transposing terms are staged through shared memory.  Units hold about
-// kTransferUnitElems elements.
+// columns (DJob), in one of three modes.  Row mode: jobs whose terms all read the
+// columns with unit stride (warp items of up to kItemElems elements: row chunks
+// x column segments).  Jobs with a transposing term: tiled mode, tiles of at
+// most 64 x 64 whose transposing terms are staged through shared memory, or for
+// small planes direct mode, every term read in place.  Units hold up to
+// kTransferUnitElems elements, fewer in transfers that would not fill the GPU.
 struct DeviceTransfer {
     std::vector<DJob> jobs;
     std::vector<DTerm> terms;
@@ -2161,24 +2161,38 @@ constexpr int32_t kTileSide = 64;          // largest tile side (elements)
 // Direct mode: planes below this many elements.  Copy P(1,0,3,2), planes of 32 x
 // 30 to 32 x 32: 155 us staged, 140 direct; of 37 x 41: 267 and 394; the four-term
 // antisymmetriser, 30 x 33: 110 and 74 us, 50 x 50: 221 and 425.
-constexpr int64_t kDirectPlane = 1024;
+// A transfer of up to kSmallTransfer elements takes it for all its planes: its
+// time is launches and the chain of one unit, and blocks on both sides of the
+// line cost two launches (transpose of 149 in blocks of 27 to 47: 6.2 us staged,
+// 10.3 in both modes, 5.2 direct).
+constexpr int64_t kDirectPlane = 1024, kSmallTransfer = 1 << 19;
 constexpr int64_t kTileSmemDoubles = 12288; // tiled mode: shared memory for all terms' tiles (96 KiB)
 
-// unit_elems: elements per unit of a large transfer; a small one has units of
-// 1024 elements or more, about 16 per SM, so that it fills the GPU.  direct:
-// transposing jobs with planes below kDirectPlane elements take the direct mode.
-DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, int64_t unit_elems = kTransferUnitElems) {
+// max_unit: elements per unit of a large transfer.  direct: transposing jobs with
+// small planes take the direct mode.
+DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, int64_t max_unit = kTransferUnitElems) {
     DeviceTransfer o;
     std::vector<DUnit> tiled_units, direct_units;
+    struct ModeJob { int32_t job; int64_t items, item_elems, elems; };
+    std::vector<ModeJob> row_jobs, tiled_jobs;
     int64_t total = 0;
+    auto add_units = [](std::vector<DUnit> &v, int32_t job, int64_t items, int64_t per_unit) {
+        for (int64_t r = 0; r < items; r += per_unit) {
+            DUnit u{};
+            u.job = job;
+            u.row_begin = r;
+            u.row_end = std::min(items, r + per_unit);
+            v.push_back(u);
+        }
+    };
     for (const TJob &j : plan.jobs) {
         int64_t n = 1;
         for (int d = 0; d < j.ndim; d++) n *= j.ext[d];
         total += n;
     }
     nsm = std::max(1, nsm);
-    unit_elems = std::min(unit_elems, std::max<int64_t>(1024, total / (16 * nsm)));
-    // row mode: likewise down to 256 elements per warp item, 64 items per SM
+    const int64_t direct_plane = !direct ? 0 : total <= kSmallTransfer ? INT64_MAX : kDirectPlane;
+    // row mode: 256 elements per warp item or more, about 64 items per SM
     const int32_t item_elems = (int32_t)std::min<int64_t>(kItemElems, std::max<int64_t>(256, total / (64 * nsm)));
     for (const TJob &j : plan.jobs) {
         const int n = j.ndim, L = n - 1;
@@ -2214,10 +2228,15 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, i
             dj.odst[dj.nout] = (int32_t)dstr[d];
             dj.nout++;
         }
-        dj.tiled = !transposing ? 0 : direct && (int64_t)dj.A * dj.B < kDirectPlane ? 2 : 1;
+        dj.tiled = !transposing ? 0 : (int64_t)dj.A * dj.B < direct_plane ? 2 : 1;
         dj.seg = dj.B > item_elems ? item_elems / 2 * 2 : dj.B;
+        // (chunks of equal length: 256 rows are two of 128, not 221 and 35: sum of
+        // two row orders in blocks of 16, order 5, 3.4e7 elements, 166 and 128 us)
         dj.nseg = (dj.B + dj.seg - 1) / dj.seg;
+        if (dj.nseg > 1) dj.seg = ((dj.B + dj.nseg - 1) / dj.nseg + 1) / 2 * 2;
         dj.ra = std::max<int32_t>(1, std::min<int32_t>(dj.A, item_elems / dj.seg));
+        dj.nra = (dj.A + dj.ra - 1) / dj.ra;
+        dj.ra = (dj.A + dj.nra - 1) / dj.nra;
         dj.nra = (dj.A + dj.ra - 1) / dj.ra;
         bool vec = !transposing && dj.seg % 2 == 0 && dj.B % 2 == 0 && dj.dst_off % 2 == 0 && dj.dq % 2 == 0;
         for (int k = 0; k < dj.nout; k++) vec = vec && dj.odst[k] % 2 == 0;
@@ -2227,10 +2246,14 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, i
         while (side > 8 && (int64_t)std::max(1, j.nterms) * side * (side + 1) > kTileSmemDoubles) side--;
         dj.nta = (dj.A + side - 1) / side;
         dj.ntb = (dj.B + side - 1) / side;
+        int64_t planes = 1;
+        for (int k = 0; k < dj.nout; k++) planes *= dj.oext[k];
         // (direct mode: down to steps of four rows where whole planes would not
-        // occupy 16 warps per SM)
+        // occupy 16 warps per SM, or the job's not the eight warps of a CTA:
+        // transpose in blocks of 28, 1.5e7 elements, 381 us with a warp per
+        // block, 163 this way, 211 staged)
         if (dj.tiled == 2) {
-            const int64_t want = std::min<int64_t>((dj.A + 3) / 4, (int64_t)dj.A * dj.B * 16 * nsm / std::max<int64_t>(1, total));
+            const int64_t want = std::min<int64_t>((dj.A + 3) / 4, std::max((7 + planes) / planes, (int64_t)dj.A * dj.B * 16 * nsm / std::max<int64_t>(1, total)));
             const int32_t rows = (int32_t)((dj.A + std::max<int64_t>(dj.nta, want) - 1) / std::max<int64_t>(dj.nta, want));
             dj.nta = (dj.A + rows - 1) / rows;               // no empty tile
         }
@@ -2278,29 +2301,38 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, i
         if (dj.tiled == 1) o.tile_bytes = std::max<int32_t>(o.tile_bytes, (toff + 1) * (int32_t)sizeof(double));
         const int32_t ji = (int32_t)o.jobs.size();
         o.jobs.push_back(dj);
-        int64_t planes = 1;
-        for (int k = 0; k < dj.nout; k++) planes *= dj.oext[k];
         if (planes * dj.A * (int64_t)dj.B >= (int64_t(1) << 31))
             throw error(kErrUnsupported, "block too large for one transfer job");
-        int64_t items, per_unit;
-        if (dj.tiled) {
-            items = planes * dj.nta * dj.ntb;
-            const int64_t tile = (int64_t)((dj.A + dj.nta - 1) / dj.nta) * ((dj.B + dj.ntb - 1) / dj.ntb);
-            // (direct mode: whole rounds of the CTA's eight warps)
-            per_unit = dj.tiled == 2 ? std::max<int64_t>(8, unit_elems / tile / 8 * 8) : std::max<int64_t>(1, unit_elems / tile);
-        } else {
-            items = planes * dj.nra * dj.nseg;
-            const int64_t item = (int64_t)dj.ra * dj.seg;
-            per_unit = std::max<int64_t>(8, (unit_elems / item + 7) / 8 * 8);
-        }
-        for (int64_t r = 0; r < items; r += per_unit) {
-            DUnit u{};
-            u.job = ji;
-            u.row_begin = r;
-            u.row_end = std::min(items, r + per_unit);
-            (dj.tiled == 2 ? direct_units : dj.tiled == 1 ? tiled_units : o.units).push_back(u);
+        const int64_t elems = planes * dj.A * (int64_t)dj.B, tile = (int64_t)ta_ext * tb_ext;
+        if (dj.tiled == 0) row_jobs.push_back({ji, planes * dj.nra * dj.nseg, (int64_t)dj.ra * dj.seg, elems});
+        if (dj.tiled == 1) tiled_jobs.push_back({ji, planes * dj.nta * dj.ntb, tile, elems});
+        if (dj.tiled == 2) {
+            // whole rounds of the CTA's eight warps, about 16 units per SM
+            const int64_t unit = std::min(max_unit, std::max<int64_t>(1024, total / (16 * nsm)));
+            add_units(direct_units, ji, planes * dj.nta * dj.ntb, std::max<int64_t>(8, unit / tile / 8 * 8));
         }
     }
+    // Row and tiled mode: CTAs take units in turn, so units of at most max_unit
+    // elements that make up whole waves, of which a job has its share rounded
+    // down.  Tiled: two CTAs per SM, and as long units as that leaves, since a
+    // unit's tiles are double-buffered (permuted copy in blocks of 27, 8.5e6
+    // elements: 45 us in 272 units, 57 in 1296; add of four terms, o=30 v=300: 224
+    // us in 2.1 waves, 208 in 3.  Eight waves or more: sum of three orders of 73^4
+    // 470 to 403 us, but of 85^4 894 to 1240).  Row: eight warps each taking an
+    // item, two rounds of eight CTAs per SM (copy P(1,0,2) in blocks of 20, 1.4e7
+    // elements: 58 us in 2704 units, 47 in 2028).
+    auto share = [&](const std::vector<ModeJob> &jobs, int64_t wave, int64_t round, std::vector<DUnit> &v) {
+        int64_t elems = 0;
+        for (const ModeJob &t : jobs) elems += t.elems;
+        const int64_t n = (elems + max_unit * wave - 1) / (max_unit * wave) * wave;
+        for (const ModeJob &t : jobs) {
+            const int64_t own = std::max<int64_t>(1, (int64_t)((double)t.elems / (double)elems * (double)n));
+            const int64_t per = std::min(std::max<int64_t>(1, max_unit / t.item_elems), (t.items + own - 1) / own);
+            add_units(v, t.job, t.items, (per + round - 1) / round * round);
+        }
+    };
+    share(row_jobs, 16 * nsm, 8, o.units);
+    share(tiled_jobs, 2 * nsm, 1, tiled_units);
     o.nrow = (int32_t)o.units.size();
     o.ntiled = (int32_t)tiled_units.size();
     o.ndirect = (int32_t)direct_units.size();
