@@ -153,9 +153,9 @@ __device__ __forceinline__ void load_stage(double *sA, double *sB, const int64_t
 // Row (column) block of a stack that holds row x: the largest R with
 // first[R] <= x.  By bisection, as a stack may have thousands of blocks: 4000
 // row blocks of 4 by 64 columns, contracted over 64, take 549 us counting up
-// from the first block (195 as one product per block), 148 this way; 48000 of
-// one row 11.3 ms (2.1) and 0.97; ladder o=32 v=48 in occupied blocks of one
-// 123 and 75 us.
+// from the first block (195 as one product per block), 90 this way with each
+// warp looking for its own blocks in the epilogue (148 with the tile's); 48000 of
+// one row 11.3 ms (2.1) and 0.54.
 __device__ __forceinline__ int block_at(const int32_t *__restrict__ first, int n, int x) {
     int lo = 0, hi = n;
     while (hi - lo > 1) {
@@ -393,15 +393,17 @@ contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict_
             continue;
         }
 
-        // the tile's part of each C block it covers (one, unless blocks of the
+        // the warp's part of each C block it covers (one, unless blocks of the
         // stack meet inside it)
-        const int R0 = block_at(rs, sk.nr, item.m0), S0 = block_at(ss, sk.ns, item.n0);
-        for (int R = R0; R < sk.nr && rs[R] < item.m0 + C::BM; R++) {
-            for (int S = S0; S < sk.ns && ss[S] < item.n0 + C::BN; S++) {
+        const int wm0 = item.m0 + wm * C::WM, wn0 = item.n0 + wn * C::WN;
+        if (wm0 >= sk.M || wn0 >= sk.N) continue;
+        const int R0 = block_at(rs, sk.nr, wm0), S0 = block_at(ss, sk.ns, wn0);
+        for (int R = R0; R < sk.nr && rs[R] < wm0 + C::WM; R++) {
+            for (int S = S0; S < sk.ns && ss[S] < wn0 + C::WN; S++) {
                 const int cblk = grid[R * sk.ns + S];
                 const DCBlock &cb = cblks[cblk];
                 // first tile row and column in the block's own numbering
-                const int mb = item.m0 + wm * C::WM + g - rs[R], nb = item.n0 + wn * C::WN + 2 * t4 - ss[S];
+                const int mb = wm0 + g - rs[R], nb = wn0 + 2 * t4 - ss[S];
                 // SCATTER: the block's destinations; else the block itself,
                 // scaled store (assign) or scaled accumulate (add)
                 int d0 = 0, d1 = 1;

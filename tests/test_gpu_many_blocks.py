@@ -61,7 +61,7 @@ def test_stacks_of_many_blocks(m, n, rows, cols, split):
 
 def test_a_stack_of_many_blocks_is_not_slower_than_its_blocks_one_by_one():
     """48000 rows as one block (51 us) and as 48000 blocks of a row: one product
-    per block takes 30 times as long (2.1 ms), a stack 19 times; counting up to
+    per block takes 30 times as long (2.1 ms), a stack 11 times; counting up to
     each tile's first block made it 223 times.  The bound has a third to spare
     over the products one by one."""
     ctx = Context(0)
