@@ -669,23 +669,29 @@ void plain_stacks(const std::vector<DTask> &dt, const std::vector<DCBlock> &dc, 
 // run or not -- a CTA of four warps alone reaches a third of it: 176 items of o=10
 // v=160 in blocks of 5 and 40 take 1182 us whole in shape 18, 784 in four chunks,
 // where one server per SM at the full rate predicts no gain.
+// What a work item takes: its multiply-adds at a resident CTA's rate, its start
+// and epilogue, and the start of each task (row offsets and the first copies of a
+// product; ladder o=12 v=16 in occupied blocks of 3, 1, 1, 1: 37 us in one chunk,
+// 17 in four); the reduction of k chunks is a launch more.
+constexpr double kItemSec = 2e-6, kTaskSec = 1e-6, kReduceLaunchSec = 4e-6;
+double cta_rate(int cfg) { return 0.8 * 40e12 / 2 / 148 * g_tile_eff[cfg] / tile_cfg_minb(cfg); }
+
 struct SplitChoice {
     size_t first;
     int sk;
     double sec;                       // estimated time of the launch
 };
 SplitChoice choose_split(int cfg, const std::vector<std::pair<double, DItem>> &v, const std::vector<int32_t> &nkt,
-                         int nsm, int split_k) {
+                         const std::vector<int32_t> &ntask, int nsm, int split_k) {
     const size_t n = v.size();
     const int bm = tile_cfg_bm(cfg), bn = tile_cfg_bn(cfg), minb = tile_cfg_minb(cfg), slots = std::max(1, nsm) * minb;
-    const double rate = 0.8 * 40e12 / 2 / 148 * g_tile_eff[cfg] / minb;      // multiply-adds per second and CTA
-    const double kBytesPerSec = 6e12, kReduceLaunchSec = 4e-6, kItemSec = 2e-6;
+    const double rate = cta_rate(cfg), kBytesPerSec = 6e12;
     auto evaluate = [&](size_t first, int sk) {
         std::vector<double> w;
         double bytes = 0;
         for (size_t i = 0; i < n; i++) {
             const int parts = i >= first ? std::max(1, std::min(sk, nkt[i])) : 1;
-            for (int p = 0; p < parts; p++) w.push_back(v[i].first / parts / rate + kItemSec);
+            for (int p = 0; p < parts; p++) w.push_back((v[i].first / rate + ntask[i] * kTaskSec) / parts + kItemSec);
             if (parts > 1) bytes += (double)(2 * parts + 1) * bm * bn * 8;
         }
         std::sort(w.rbegin(), w.rend());
@@ -730,12 +736,13 @@ void append_launch(int cfg, std::vector<std::pair<double, DItem>> &v, const std:
     });
     const int bm = tile_cfg_bm(cfg), bn = tile_cfg_bn(cfg), bk = tile_cfg_bk(cfg);
     const size_t n = v.size();
-    std::vector<int32_t> nkt(n, 0);
+    std::vector<int32_t> nkt(n, 0), ntask(n, 0);
     for (size_t i = 0; i < n; i++) {
         const DCBlock &b = dc[ps.first_block(v[i].second.stack)];
+        ntask[i] = b.t_end - b.t_begin;
         for (int32_t t = b.t_begin; t < b.t_end; t++) nkt[i] += (dt[t].K + bk - 1) / bk;
     }
-    const SplitChoice choice = choose_split(cfg, v, nkt, nsm, split_k);
+    const SplitChoice choice = choose_split(cfg, v, nkt, ntask, nsm, split_k);
     const size_t first_split = choice.first;
     const int sk = choice.sk;
     DmmaLaunch L;
@@ -842,14 +849,66 @@ void plain_task_arrays(const ltg_plan *pl, int64_t c_elems, const std::vector<Ge
     }
 }
 
+// The one shape in which products whose tiles would not occupy every SM finish
+// first, by the number of tiles, their k chunks and the time of the longest.
+// pick_tile's least padded work takes large tiles in few CTAs there, and a
+// launch, with its tail, for each shape it picks: ladder o=12 v=18 in blocks of 6,
+// 5 and 4, 17 us one product per block, 42 stacked in two shapes, 15 in one of
+// 32 x 32; o=12 v=48 in blocks of 4, 2 and 24 39, 55 and 20 us.
+struct SmallProduct {
+    int64_t M, N;
+    double K;
+    int32_t ntask;
+};
+int pick_small(const std::vector<SmallProduct> &v, int nsm, int split_k) {
+    int best = 0;
+    double bestt = 1e300;
+    for (int c = 0; c < kNumShapes; c++) {
+        const int bm = tile_cfg_bm(c), bn = tile_cfg_bn(c);
+        const int64_t ctas = (int64_t)std::max(1, nsm) * tile_cfg_minb(c);
+        double longest = 0;
+        int64_t n = 0;
+        for (const SmallProduct &p : v) {
+            n += ((p.M + bm - 1) / bm) * ((p.N + bn - 1) / bn);
+            // (a task's last k tile is half empty on the mean)
+            longest = std::max(longest, (double)bm * bn * (p.K + 0.5 * p.ntask * tile_cfg_bk(c)) / cta_rate(c) + p.ntask * kTaskSec);
+        }
+        for (int parts = split_k >= 1 ? split_k : 1; parts <= (split_k >= 1 ? split_k : 4); parts++) {
+            const double t = (double)((n * parts + ctas - 1) / ctas) * (longest / parts + kItemSec) + (parts > 1 ? kReduceLaunchSec : 0.0);
+            if (t < bestt) { bestt = t; best = c; }
+        }
+    }
+    return best;
+}
+
+// Tile shapes of products: pick_tile's, or pick_small's for all if these would
+// leave SMs without a tile.
+std::vector<int> pick_tiles(const std::vector<SmallProduct> &v, int nsm, int split_k) {
+    std::vector<int> cfgs;
+    int64_t tiles = 0;
+    for (const SmallProduct &p : v) {
+        const int c = pick_tile(p.M, p.N, p.K);
+        cfgs.push_back(c);
+        tiles += ((p.M + tile_cfg_bm(c) - 1) / tile_cfg_bm(c)) * ((p.N + tile_cfg_bn(c) - 1) / tile_cfg_bn(c));
+    }
+    if (tiles < nsm) std::fill(cfgs.begin(), cfgs.end(), pick_small(v, nsm, split_k));
+    return cfgs;
+}
+
 // Work items of the stacks by tile shape: the plan's forced or autotuned shape,
-// or pick_tile's.
-void stack_items(const ltg_plan *pl, const PlainStacks &ps, const std::vector<CBlockTask> &cbt,
+// or pick_tiles'.
+void stack_items(const ltg_plan *pl, const PlainStacks &ps, const std::vector<CBlockTask> &cbt, int split_k,
                  std::vector<std::vector<std::pair<double, DItem>>> &per_cfg) {
+    std::vector<SmallProduct> v;
+    for (size_t k = 0; k < ps.stacks.size(); k++) {
+        const CBlockTask &b = cbt[ps.first_block((int32_t)k)];
+        v.push_back({ps.stacks[k].M, ps.stacks[k].N, b.kflops, b.t_end - b.t_begin});
+    }
+    const std::vector<int> cfgs = pick_tiles(v, pl->ctx->nsm, split_k);
     for (size_t k = 0; k < ps.stacks.size(); k++) {
         const DStack &st = ps.stacks[k];
         const CBlockTask &b = cbt[ps.first_block((int32_t)k)];
-        int cfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(st.M, st.N, b.kflops);
+        int cfg = pl->forced_tile >= 0 ? pl->forced_tile : cfgs[k];
         auto ov = pl->tile_override.find({st.M, st.N});
         if (pl->forced_tile < 0 && ov != pl->tile_override.end()) cfg = ov->second;
         const int bm = tile_cfg_bm(cfg), bn = tile_cfg_bn(cfg);
@@ -889,7 +948,7 @@ ContractExec *prepare_exec(ltg_plan *pl, ltg_bt *c, double ka, double kb, double
     PlainStacks ps;
     plain_stacks(dt, dc, use, ps);
     std::vector<std::vector<std::pair<double, DItem>>> per_cfg(kNumShapes);
-    stack_items(pl, ps, cbt, per_cfg);
+    stack_items(pl, ps, cbt, pl->split_k, per_cfg);
     std::vector<DItem> items;
     std::vector<DSplit> splits;
     int64_t ws_elems = 0;
@@ -1528,16 +1587,17 @@ void build_plain_groups(ltg_plan *pl, const BlockTensorHost &ch, const std::vect
     {
         int64_t o2 = 0;
         double best = -1;
+        size_t costliest = 0;
+        std::vector<SmallProduct> v;
         for (const CrtGroupHost &G : groups) {
             if (!plain_group_layout(G, o2, lay)) { group_of.assign(cbt.size(), -1); return; }
             const double w = (double)lay.rows * lay.cols * lay.kt;
-            if (w > best) {
-                best = w;
-                gcfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tile(lay.rows, lay.cols, (double)lay.kt);
-                auto ov = pl->tile_override.find({lay.rows, lay.cols});
-                if (pl->forced_tile < 0 && ov != pl->tile_override.end()) gcfg = ov->second;
-            }
+            if (w > best) { best = w; costliest = v.size(); }
+            v.push_back({lay.rows, lay.cols, (double)lay.kt, 1});
         }
+        gcfg = pl->forced_tile >= 0 ? pl->forced_tile : pick_tiles(v, pl->ctx->nsm, pl->split_k)[costliest];
+        auto ov = pl->tile_override.find({v[costliest].M, v[costliest].N});
+        if (pl->forced_tile < 0 && ov != pl->tile_override.end()) gcfg = ov->second;
     }
     for (size_t gi = 0; gi < groups.size(); gi++) {
         const CrtGroupHost &G = groups[gi];
@@ -3064,7 +3124,7 @@ SymExec *prepare_sym(ltg_plan *pl, ltg_bt *r, int32_t mode, int32_t L, double c,
     PlainStacks ps;
     plain_stacks(dt, dc, use, ps);
     std::vector<std::vector<std::pair<double, DItem>>> per_cfg(kNumShapes);
-    stack_items(pl, ps, cbt, per_cfg);
+    stack_items(pl, ps, cbt, 1, per_cfg);
     std::vector<DItem> items;
     std::vector<DSplit> splits;
     int64_t ws_elems = 0;
