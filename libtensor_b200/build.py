@@ -24,12 +24,16 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
               "--expt-relaxed-constexpr", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-Wall", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
 
+# Sources; (source, object, defines) where one source makes several objects.
 SOURCES = [
     "ltg_host.cpp",
     "ltg_capi.cu",
     "contract_fp64.cu",
     "elementwise.cu",
     "ozaki.cu",
+    ("ozaki.cu", "ozaki_int8.o", ["-DLTG_OZ_KIND=0"]),
+    ("ozaki.cu", "ozaki_bf16.o", ["-DLTG_OZ_KIND=1"]),
+    ("ozaki.cu", "ozaki_fp8.o", ["-DLTG_OZ_KIND=2"]),
     "noalloc.cu",
     "crt.cu",
     "group.cu",
@@ -44,13 +48,13 @@ def _nvcc():
     raise RuntimeError("nvcc not found")
 
 
-def _compile(src, obj, verbose):
+def _compile(src, obj, defines, verbose):
     path = os.path.join(CSRC, src)
     t_src = os.path.getmtime(path)
     if src.endswith(".cpp"):
         cmd = [os.environ.get("CXX", "g++"), *CXX_FLAGS, "-I/usr/local/cuda/include", "-c", path, "-o", obj]
     else:
-        cmd = [_nvcc(), *ARCH, *NVCC_FLAGS, "-c", path, "-o", obj]
+        cmd = [_nvcc(), *ARCH, *NVCC_FLAGS, *defines, "-c", path, "-o", obj]
     if verbose:
         print(" ".join(cmd), flush=True)
     r = subprocess.run(cmd, capture_output=True, text=True)
@@ -77,12 +81,13 @@ def build(verbose=False, force=False):
     jobs = []
     objs = []
     for s in srcs:
-        obj = os.path.join(BUILD, s.rsplit(".", 1)[0] + ".o")
+        s, obj, defines = (s, s.rsplit(".", 1)[0] + ".o", []) if isinstance(s, str) else s
+        obj = os.path.join(BUILD, obj)
         objs.append(obj)
         if force or _stale(obj, [os.path.join(CSRC, s), *headers]):
-            jobs.append((s, obj))
+            jobs.append((s, obj, defines))
     with cf.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
-        for f in [ex.submit(_compile, s, o, verbose) for s, o in jobs]:
+        for f in [ex.submit(_compile, s, o, d, verbose) for s, o, d in jobs]:
             f.result()
     if jobs or not os.path.exists(LIB):
         # --no-undefined: an object compiled from an older source (a changed

@@ -49,6 +49,7 @@
 namespace ltg {
 
 // k elements per 32-byte k block: 32 for 8-bit slices, 16 for BF16.
+#ifndef LTG_OZ_KIND
 void oz_kind_params(int kind, int *beta0, int *beta, int *esz, int *kbe, int64_t *maxprod) {
     switch (kind) {
     case kOzInt8: *beta0 = 6; *beta = 7; *esz = 1; *kbe = 32; *maxprod = 64 * 64; break;
@@ -56,6 +57,33 @@ void oz_kind_params(int kind, int *beta0, int *beta, int *esz, int *kbe, int64_t
     default:      *beta0 = 4; *beta = 5; *esz = 1; *kbe = 32; *maxprod = 16 * 16; break;
     }
 }
+#endif
+
+// What one slice-products launch takes besides its template arguments.
+struct OzGemmArgs {
+    const DPanel *panels;
+    const uint8_t *slices;
+    const DOzTask *tasks;
+    const DCBlock *cblks;
+    const DOzItem *items;
+    int32_t nitems;
+    const int32_t *exps;
+    double *c;
+    int32_t add, swap, chunk_kb, max_nt;
+    int32_t *err;
+    uint64_t wait_ns;
+    cudaStream_t s;
+    const int2 *drange;
+    const DCBlock *dests;
+};
+
+// The kernels of one kind.  Each kind is a translation unit of its own (compiled
+// with LTG_OZ_KIND set to it), as this file's 51 kernels take several minutes
+// one after the other; the unit without LTG_OZ_KIND holds the entry points.
+template<int KIND> cudaError_t oz_launch_gemm(int S, const OzGemmArgs &a);
+template<int KIND> cudaError_t oz_launch_split(int S, const DPanel *panels, const int4 *units, int32_t nunits,
+                                               const double *a, const double *b, uint8_t *slices, int32_t *exps,
+                                               cudaStream_t s);
 
 namespace {
 
@@ -732,24 +760,6 @@ oz_gemm_kernel(const DPanel *__restrict__ panels, const uint8_t *__restrict__ sl
 
 int g_nsm = 0;
 
-// What one slice-products launch takes besides its template arguments.
-struct OzGemmArgs {
-    const DPanel *panels;
-    const uint8_t *slices;
-    const DOzTask *tasks;
-    const DCBlock *cblks;
-    const DOzItem *items;
-    int32_t nitems;
-    const int32_t *exps;
-    double *c;
-    int32_t add, swap, chunk_kb, max_nt;
-    int32_t *err;
-    uint64_t wait_ns;
-    cudaStream_t s;
-    const int2 *drange;
-    const DCBlock *dests;
-};
-
 template<int KIND, int S, bool SCATTER = false>
 cudaError_t launch_gemm_s(const OzGemmArgs &a) {
     int beta0, beta, esz, kbe;
@@ -783,16 +793,6 @@ cudaError_t launch_gemm_s(const OzGemmArgs &a) {
     return cudaGetLastError();
 }
 
-template<int KIND>
-cudaError_t launch_gemm_k(int S, const OzGemmArgs &a) {
-    switch (S) {
-#define CASE_S(n) case n: return launch_gemm_s<KIND, n>(a);
-    CASE_S(1) CASE_S(2) CASE_S(3) CASE_S(4) CASE_S(5) CASE_S(6) CASE_S(7) CASE_S(8)
-#undef CASE_S
-    default: return cudaErrorInvalidValue;
-    }
-}
-
 // Clocks per k block of one 128 x nt tile: its S(S+1)/2 products at nt / 2
 // clocks each, or its operand images from L2 at kL2Bytes per clock and SM
 // (about 11.6 TB/s over the chip), whichever is longer.  The rule takes nt = 112
@@ -806,6 +806,39 @@ double oz_tile_clocks(int nt, int S) {
 }
 
 }  // namespace
+
+#ifdef LTG_OZ_KIND
+
+template<int KIND>
+cudaError_t oz_launch_gemm(int S, const OzGemmArgs &a) {
+    // the scattering form for the kind's default slice count only
+    constexpr int kScatter = KIND == kOzE4m3 ? 8 : 7;
+    if (a.dests) return S == kScatter ? launch_gemm_s<KIND, kScatter, true>(a) : cudaErrorNotSupported;
+    switch (S) {
+#define CASE_S(n) case n: return launch_gemm_s<KIND, n>(a);
+    CASE_S(1) CASE_S(2) CASE_S(3) CASE_S(4) CASE_S(5) CASE_S(6) CASE_S(7) CASE_S(8)
+#undef CASE_S
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+template<int KIND>
+cudaError_t oz_launch_split(int S, const DPanel *panels, const int4 *units, int32_t nunits, const double *a,
+                            const double *b, uint8_t *slices, int32_t *exps, cudaStream_t s) {
+    switch (S) {
+#define CASE_S(n) case n: oz_split_kernel<KIND, n><<<nunits, kSplitThreads, 0, s>>>(panels, units, a, b, slices, exps); break;
+    CASE_S(1) CASE_S(2) CASE_S(3) CASE_S(4) CASE_S(5) CASE_S(6) CASE_S(7) CASE_S(8)
+#undef CASE_S
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+template cudaError_t oz_launch_gemm<LTG_OZ_KIND>(int, const OzGemmArgs &);
+template cudaError_t oz_launch_split<LTG_OZ_KIND>(int, const DPanel *, const int4 *, int32_t, const double *,
+                                                  const double *, uint8_t *, int32_t *, cudaStream_t);
+
+#else
 
 int32_t oz_tile_width(int64_t rows, int S) {
     int32_t best = 16;
@@ -832,15 +865,9 @@ int oz_split_unit_rows(int K) {
 cudaError_t launch_oz_split(int kind, const DPanel *panels, const int4 *units, int32_t nunits, const double *a,
                             const double *b, uint8_t *slices, int32_t *exps, int32_t S, cudaStream_t s) {
     if (nunits <= 0) return cudaSuccess;
-    switch (kind * 16 + S) {
-#define CASE_KS(k, n) case k * 16 + n: oz_split_kernel<k, n><<<nunits, kSplitThreads, 0, s>>>(panels, units, a, b, slices, exps); break;
-#define CASE_K(k) CASE_KS(k, 1) CASE_KS(k, 2) CASE_KS(k, 3) CASE_KS(k, 4) CASE_KS(k, 5) CASE_KS(k, 6) CASE_KS(k, 7) CASE_KS(k, 8)
-    CASE_K(kOzInt8) CASE_K(kOzBf16) CASE_K(kOzE4m3)
-#undef CASE_K
-#undef CASE_KS
-    default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    if (kind == kOzInt8) return oz_launch_split<kOzInt8>(S, panels, units, nunits, a, b, slices, exps, s);
+    if (kind == kOzBf16) return oz_launch_split<kOzBf16>(S, panels, units, nunits, a, b, slices, exps, s);
+    return oz_launch_split<kOzE4m3>(S, panels, units, nunits, a, b, slices, exps, s);
 }
 
 cudaError_t launch_oz_gemm(int kind, const DPanel *panels, const uint8_t *slices, const DOzTask *tasks,
@@ -850,16 +877,11 @@ cudaError_t launch_oz_gemm(int kind, const DPanel *panels, const uint8_t *slices
     if (S < 1 || S > 8 || max_nt > oz_max_nt(S)) return cudaErrorInvalidValue;
     const OzGemmArgs a{panels, slices, tasks, cblks, items, nitems, exps, c, add, swap, chunk_kb, max_nt,
                        err, wait_ns, s, drange, dests};
-    if (dests) {
-        // the scattering form for each kind's default slice count only
-        if (kind == kOzInt8 && S == 7) return launch_gemm_s<kOzInt8, 7, true>(a);
-        if (kind == kOzBf16 && S == 7) return launch_gemm_s<kOzBf16, 7, true>(a);
-        if (kind == kOzE4m3 && S == 8) return launch_gemm_s<kOzE4m3, 8, true>(a);
-        return cudaErrorNotSupported;
-    }
-    if (kind == kOzInt8) return launch_gemm_k<kOzInt8>(S, a);
-    if (kind == kOzBf16) return launch_gemm_k<kOzBf16>(S, a);
-    return launch_gemm_k<kOzE4m3>(S, a);
+    if (kind == kOzInt8) return oz_launch_gemm<kOzInt8>(S, a);
+    if (kind == kOzBf16) return oz_launch_gemm<kOzBf16>(S, a);
+    return oz_launch_gemm<kOzE4m3>(S, a);
 }
+
+#endif
 
 }  // namespace ltg
