@@ -1,5 +1,5 @@
-"""Plain FP64 contractions that do not fill the GPU: the tile shape and k chunks
-the plan picks by itself against every shape forced on it."""
+"""Plain FP64 contractions that do not fill the GPU, or are short: the tile shape
+and k chunks the plan picks by itself against every shape forced on it."""
 import numpy as np
 import pytest
 
@@ -60,6 +60,28 @@ def test_picked_shape_is_near_the_best(make):
         op.set_tile(tile)
         best = min(best, _us(ctx, lambda: op.perform(C)))
     assert own <= 1.6 * best + 4.0, (own, best)
+    for x in (op, C, A, B):
+        x.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("k", [64, 160, 220])
+def test_picked_shape_of_short_contractions(k):
+    """1500 x 1500 over k: within 1.25 of the fastest of the shapes with two CTAs
+    per SM.  Measured 1.07 at 80; a shape for contractions below 256, chosen on one
+    size, took 1.22 at 160 and 1.32 at 220."""
+    ctx = Context(0)
+    A, B, contr = _matrices(ctx, [1500], [1500], [k])
+    A.fill_seeded(1, 1.0)
+    B.fill_seeded(2, 1.0)
+    op = btod_contract2(contr, A, B)
+    C = op.make_result()
+    own = _us(ctx, lambda: op.perform(C))
+    best = 1e30
+    for tile in range(17, 22):
+        op.set_tile(tile)
+        best = min(best, _us(ctx, lambda: op.perform(C)))
+    assert own <= 1.25 * best, (own, best)
     for x in (op, C, A, B):
         x.close()
     ctx.close()
