@@ -51,15 +51,14 @@ constexpr int kSubBytes = 2 * kXTile + kMaxNt * kKB;    // one k block: two M ti
 constexpr int kMaxStages = 8;
 // Four epilogue warps per TMEM lane quarter: with two, reading back a modulus
 // (2 x 128 x 208 sums, 5,700 clocks) held the ring's short products for 41 % of
-// their time; four run the ring in 143 us (148), the ladder o=40 v=240 in 1.74 ms
-// (1.76).
+// their time; four run the ring's products in 143 us (148), the ladder's at o=40
+// v=240 in 1.74 ms (1.76: 1 % of the kernel, less than runs of the call differ).
 constexpr int kEpiWarps = 16;
 constexpr int kGemmThreads = 32 * (kEpiWarps + 2);  // + bulk-copy producer + MMA issuer
 constexpr uint64_t kWaitNs = 2000000000ull;         // 2 s: the drain waits after an abort
 constexpr double kMagicD = 6755399441055744.0;      // 1.5 * 2^52: round-to-integer constant
 constexpr int32_t kNoExp = -1000000;                // exponent of a row with no non-zero element
 constexpr int32_t kKeepRow = -2000000;              // redo pass: a row whose residues stand
-constexpr int32_t kRereadRow = 1000000;             // exponent pass: a row with a NaN or an infinity
 
 // The moduli (pairwise coprime, <= 256) and the constants derived from them,
 // as compile-time functions so that unrolled loops over the moduli fold them
@@ -191,30 +190,30 @@ __device__ __forceinline__ int64_t koffset(const DCrtPanel &P, int mode, const i
 // for 78 MB, 20 this way with two 32-byte groups in flight; more of them cost the
 // core tiles of short rows their occupancy; ring D2h 71 to 68 us).
 // NaNs and infinities take no part: integers cannot carry them, so what reads
-// one means nothing, but the row's other elements keep their scale.  A row
-// whose maximum comes out non-finite is read again without them, so that the
-// pass has no test per element.
+// one means nothing, but the row's other elements keep their scale.  The high
+// words are compared as signed numbers plus kHiBias, which makes those of a NaN
+// or an infinity negative: an add and a maximum in one instruction (ring D2h:
+// 67.1 us without, 68.5 with a test per element, 67.2 this way).
 constexpr uint32_t kInfHi = 0x7ff00000u;                // high word of an infinity
+constexpr int kHiBias = 1 << 20;
 __device__ __forceinline__ uint32_t magnitude_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
 struct RowMax {
-    uint32_t hi = 0, lo = 0;
+    int hb = kHiBias;
+    uint32_t lo = 0;
     __device__ __forceinline__ void take(double x) {
-        hi = max(hi, magnitude_hi(x));
+        hb = __viaddmax_s32((int)magnitude_hi(x), kHiBias, hb);
         lo |= (uint32_t)__double2loint(x);
     }
-    __device__ __forceinline__ void take_finite(double x) {
-        if (magnitude_hi(x) < kInfHi) take(x);
-    }
-    __device__ __forceinline__ bool finite() const { return hi < kInfHi; }
     __device__ __forceinline__ void join(int lanes) {
-        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, lanes));
+        hb = max(hb, __shfl_xor_sync(0xffffffffu, hb, lanes));
         lo |= __shfl_xor_sync(0xffffffffu, lo, lanes);
     }
+    __device__ __forceinline__ bool any() const { return (hb - kHiBias) != 0 || lo != 0; }
     // e with |x| in [2^(e-1), 2^e), or kNoExp without a non-zero element
     __device__ __forceinline__ int exponent() const {
-        if ((hi | lo) == 0) return kNoExp;
+        if (!any()) return kNoExp;
         int e;
-        frexp(__hiloint2double((int)hi, (int)lo), &e);
+        frexp(__hiloint2double(hb - kHiBias, (int)lo), &e);
         return e;
     }
 };
@@ -280,18 +279,7 @@ crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
             m.join(1);
             m.join(2);
             m.join(4);
-            if (__any_sync(0xffffffffu, !m.finite())) {
-                RowMax f;
-                if (valid)
-#pragma unroll 1
-                    for (int k0 = 4 * c; k0 < K; k0 += step)
-                        for (int j = 0; j < 4 && k0 + j < K; j++) f.take_finite(row[koffset(P, mode, koff, k0 + j)]);
-                f.join(1);
-                f.join(2);
-                f.join(4);
-                if (!m.finite()) m = f;
-            }
-            if (valid && c == 0 && (m.hi | m.lo) != 0)
+            if (valid && c == 0 && m.any())
                 atomicMax(&tab[gidx[P.g_off + r]], m.exponent() + (smp ? 1 : 0));      // one binade of headroom
             continue;
         }
@@ -303,8 +291,7 @@ crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
         auto flush = [&]() {
             m.join(1);
             m.join(2);
-            if (kq == 0 && (m.hi | m.lo) != 0)
-                atomicMax(&rexp[cur * 8 + lrow], m.finite() ? m.exponent() : kRereadRow);
+            if (kq == 0 && m.any()) atomicMax(&rexp[cur * 8 + lrow], m.exponent());
             m = RowMax();
         };
         while (kt >= nkt) { kt -= nkt; rg++; }
@@ -327,15 +314,7 @@ crt_exp_kernel(const DCrtPanel *__restrict__ panels, const int4 *__restrict__ un
         __syncthreads();
         for (int i = threadIdx.x; i < un.z; i += blockDim.x) {
             const int r = un.y + i;
-            if (r >= P.rows || rexp[i] == kNoExp) continue;
-            int e = rexp[i];
-            if (e == kRereadRow) {
-                RowMax f;
-#pragma unroll 1
-                for (int k = 0; k < K; k++) f.take_finite(src[roff[i] + koffset(P, mode, koff, k)]);
-                e = f.exponent();
-            }
-            if (e > kNoExp) atomicMax(&tab[gidx[P.g_off + r]], e);
+            if (r < P.rows && rexp[i] > kNoExp) atomicMax(&tab[gidx[P.g_off + r]], rexp[i]);
         }
     }
 }
@@ -894,8 +873,8 @@ crt_gemm_kernel(const DCrtPanel *__restrict__ panels, const uint8_t *__restrict_
                             const uint32_t dx = desc_lo(smem0 + st * (KB * kSubBytes));
                             const uint32_t dy = dx + (uint32_t)((2 * KB * kXTile) >> 4);
                             // whole stages without a branch or a descriptor built
-                            // per MMA: ladder o=40 v=240 1.77 ms in the general
-                            // form, 1.73 this way
+                            // per MMA: products of the ladder o=40 v=240 1.77 ms in
+                            // the general form, 1.73 this way
                             if (item.nx == 2 && nsub == KB) {
 #pragma unroll
                                 for (int j = 0; j < KB; j++) {
