@@ -158,11 +158,12 @@ __device__ __forceinline__ void load_stage(double *sA, double *sB, const int64_t
 // one row 11.3 ms (2.1) and 0.54.
 __device__ __forceinline__ int block_at(const int32_t *__restrict__ first, int n, int x) {
     int lo = 0, hi = n;
-    while (hi - lo > 1) {
+    while (hi - lo > 4) {
         const int mid = (lo + hi) >> 1;
         if (first[mid] <= x) lo = mid;
         else hi = mid;
     }
+    while (lo + 1 < hi && first[lo + 1] <= x) lo++;
     return lo;
 }
 
@@ -394,12 +395,12 @@ contract_fp64_kernel(const DTask *__restrict__ tasks, const DCBlock *__restrict_
         }
 
         // the warp's part of each C block it covers (one, unless blocks of the
-        // stack meet inside it)
-        const int wm0 = item.m0 + wm * C::WM, wn0 = item.n0 + wn * C::WN;
-        if (wm0 >= sk.M || wn0 >= sk.N) continue;
-        const int R0 = block_at(rs, sk.nr, wm0), S0 = block_at(ss, sk.ns, wn0);
-        for (int R = R0; R < sk.nr && rs[R] < wm0 + C::WM; R++) {
-            for (int S = S0; S < sk.ns && ss[S] < wn0 + C::WN; S++) {
+        // stack meet inside it; past the stack the last one, which has no such
+        // rows); the shuffles tell the compiler that the bounds are the warp's, and
+        // the loops stay out of the accumulators' registers
+        const int wm0 = __shfl_sync(0xffffffffu, item.m0 + wm * C::WM, 0), wn0 = __shfl_sync(0xffffffffu, item.n0 + wn * C::WN, 0);
+        for (int R = block_at(rs, sk.nr, wm0); R < sk.nr && rs[R] < wm0 + C::WM; R++) {
+            for (int S = block_at(ss, sk.ns, wn0); S < sk.ns && ss[S] < wn0 + C::WN; S++) {
                 const int cblk = grid[R * sk.ns + S];
                 const DCBlock &cb = cblks[cblk];
                 // first tile row and column in the block's own numbering
