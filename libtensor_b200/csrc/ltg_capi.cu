@@ -696,9 +696,11 @@ SplitChoice choose_split(int cfg, const std::vector<std::pair<double, DItem>> &v
             for (int p = 0; p < parts; p++) w.push_back((v[i].first / rate + ntask[i] * kTaskSec) / parts + kItemSec);
             if (parts > 1) bytes += (double)(2 * parts + 1) * bm * bn * 8;
         }
+        // (no more chunks than CTAs: the longest)
+        if (w.size() <= (size_t)slots)
+            return *std::max_element(w.begin(), w.end()) + (bytes > 0 ? bytes / kBytesPerSec + kReduceLaunchSec : 0.0);
         std::sort(w.rbegin(), w.rend());
-        std::priority_queue<double, std::vector<double>, std::greater<double>> load;
-        for (int k = 0; k < slots; k++) load.push(0.0);
+        std::priority_queue<double, std::vector<double>, std::greater<double>> load(std::greater<double>(), std::vector<double>(slots, 0.0));
         double mk = 0;
         for (double x : w) {
             double t = load.top() + x;
