@@ -2238,7 +2238,7 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, i
     DeviceTransfer o;
     std::vector<DUnit> tiled_units, direct_units;
     struct ModeJob { int32_t job; int64_t items, item_elems, elems; };
-    std::vector<ModeJob> row_jobs, tiled_jobs;
+    std::vector<ModeJob> row_jobs, tiled_jobs, small_jobs;
     int64_t total = 0;
     auto add_units = [](std::vector<DUnit> &v, int32_t job, int64_t items, int64_t per_unit) {
         for (int64_t r = 0; r < items; r += per_unit) {
@@ -2369,7 +2369,7 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, i
             throw error(kErrUnsupported, "block too large for one transfer job");
         const int64_t elems = planes * dj.A * (int64_t)dj.B, tile = (int64_t)ta_ext * tb_ext;
         if (dj.tiled == 0) row_jobs.push_back({ji, planes * dj.nra * dj.nseg, (int64_t)dj.ra * dj.seg, elems});
-        if (dj.tiled == 1) tiled_jobs.push_back({ji, planes * dj.nta * dj.ntb, tile, elems});
+        if (dj.tiled == 1) (direct || tile >= kDirectPlane ? tiled_jobs : small_jobs).push_back({ji, planes * dj.nta * dj.ntb, tile, elems});
         if (dj.tiled == 2) {
             // whole rounds of the CTA's eight warps, about 16 units per SM
             const int64_t unit = std::min(max_unit, std::max<int64_t>(1024, total / (16 * nsm)));
@@ -2397,6 +2397,10 @@ DeviceTransfer device_transfer(const TransferPlan &plan, int nsm, bool direct, i
     };
     share(row_jobs, 16 * nsm, 8, o.units);
     share(tiled_jobs, 2 * nsm, 1, tiled_units);
+    // (the dot product stages small planes too: their barriers and latencies are
+    // what takes the time, and more CTAs fit; o=20 v=52 in blocks of 7 to 18, 122 us
+    // in one wave of 296, 57 in 1184)
+    share(small_jobs, 8 * nsm, 1, tiled_units);
     o.nrow = (int32_t)o.units.size();
     o.ntiled = (int32_t)tiled_units.size();
     o.ndirect = (int32_t)direct_units.size();
