@@ -201,7 +201,7 @@ struct RowMax {
     int hb = kHiBias;
     uint32_t lo = 0;
     __device__ __forceinline__ void take(double x) {
-        hb = __viaddmax_s32((int)magnitude_hi(x), kHiBias, hb);
+        hb = max((int)(magnitude_hi(x) + (uint32_t)kHiBias), hb);
         lo |= (uint32_t)__double2loint(x);
     }
     __device__ __forceinline__ void join(int lanes) {
