@@ -1,5 +1,7 @@
 """Workspace of the k-split partial tiles: shared by the plans of a context and
 given back with them."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -28,6 +30,7 @@ def test_workspace_goes_with_its_plans():
     """Four chunks of every tile of a 4096 x 4096 result are 512 MB; a second
     plan shares them, the first may go, and with the last plan they go too (but
     for 32 MB the context keeps, and 16 MB for what the driver rounds to)."""
+    gc.collect()                                 # nothing of other tests is freed meanwhile
     ctx = Context(0)
     rng = np.random.default_rng(1)
     x = rng.standard_normal((4096, 256))
