@@ -534,7 +534,8 @@ int32_t vec16_ok(int64_t off, const SubDims &rows, const SubDims &k, bool second
 constexpr int kNumShapes = 22;
 // Relative rates of the shapes per padded element.  The m8n8k4 shapes with two
 // CTAs per SM (17-21) from the ladder o=40 v=240 (10.39 ms in shape 18, 10.47 in
-// 19, 10.96 in 20, 11.10 in 17, whose 64-row tiles pad 400 rows to 448), the
+// 19, 10.96 in 20, 11.10 in 17; 17 and 20 pad 400 rows to 448, which is taken out
+// of their rates, as pick_tile counts it), the
 // others from the same runs (11: 11.65, 16: 11.89, 12: 11.95) and from shorter
 // rows (8, 9, 3: blocks of 16, 32 and 25 rows).
 double g_tile_eff[kNumShapes] = {0.80, 0.60, 0.75, 0.35, 0.87, 0.80, 0.70, 0.85, 0.45, 0.60, 0.88, 0.89,
